@@ -42,6 +42,10 @@ struct Material {
   double c3, c4, c5, c6;  // data_mod.f90:104-107
 };
 
+// Device workspaces of a call that a context keeps for its next one: at most this many
+// bytes each, larger ones are released when the call ends.
+constexpr size_t kWsKeep = size_t(512) << 20;
+
 inline Material make_material(double mu, double nu) {
   Material m;
   m.mu = mu;
@@ -81,6 +85,18 @@ struct DBuf {
   }
   size_t bytes() const { return count * sizeof(T); }
 };
+
+// 1 / sqrt(x) from the hardware's approximation of its leading bits and one third-order
+// step: with y (1 + d) = 1 / sqrt(x) and e = 1 - x y^2, y (1 + e/2 + 3/8 e^2) is off by
+// 5/16 e^3, below rounding for the approximation's |e| < 2^-18.  Five FP64 operations; no
+// subnormal or infinite arguments (squared distances).
+__device__ __forceinline__ double rsqrt_h3(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+__device__ __forceinline__ float rsqrt_h3(float x) { return rsqrtf(x); }
 
 // One-time set-up that CUDA keeps per device (kernel attributes, __constant__ tables),
 // tracked per device so that a process driving several GPUs sets up each of them:
@@ -223,7 +239,10 @@ struct bem_ctx {
   int panel_width = 0;  // FP32 factorisation panel width of the *_IR modes (0: the mode's own)
   int f32_gemm_override = -1;  // BEM_F32_GEMM environment override (0, 1, 3)
   // tcgen05 trailing update: BF16 hi/lo operand copies and its error word
-  bem::DBuf<unsigned long long> ip_counters;  // internal points: far and near evaluations
+  // internal points: the tables, partial sums and pair lists of a call, and the pairs'
+  // sums; kept up to kWsKeep bytes each for the next call
+  bem::DBuf<unsigned char> ip_ws, ip_pairs;
+  bem::DBuf<double> ip_io;  // the host interface's device copies, kept likewise
   bem::DBuf<unsigned char> umma_buf;
   bem::DBuf<int> umma_err;
   // profiling (bem_profile_begin/end)

@@ -544,21 +544,24 @@ int bem_internal_points(bem_ctx* c, int l, const double* cx, const double* cy, c
   if (l == 0) return BEM_OK;
   if (!cx || !cy || !cz || !u || !s || !pr || !vm) return bem_fail(c, BEM_ERR_ARG, "internal_points: null");
   BEM_CUDA(c, cudaSetDevice(c->device));
-  bem::DBuf<double> d;
-  BEM_CUDA(c, d.alloc(16 * (size_t)l));
-  double* p = d.p;
+  if (c->ip_io.count < 16 * (size_t)l) BEM_CUDA(c, c->ip_io.alloc(16 * (size_t)l));
+  double* p = c->ip_io.p;
   double *dx = p, *dy = p + l, *dz = p + 2 * (size_t)l, *du = p + 3 * (size_t)l, *ds = p + 6 * (size_t)l,
          *dp = p + 12 * (size_t)l, *dv = p + 15 * (size_t)l;
   BEM_CUDA(c, cudaMemcpyAsync(dx, cx, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(dy, cy, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(dz, cz, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   int rc = bem::launch_internal_points(c, l, dx, dy, dz, du, ds, dp, dv, flags);
-  if (rc) return rc;
+  if (rc) {
+    if (c->ip_io.bytes() > bem::kWsKeep) c->ip_io.release();
+    return rc;
+  }
   BEM_CUDA(c, cudaMemcpyAsync(u, du, 3 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(s, ds, 6 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(pr, dp, 3 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(vm, dv, (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (c->ip_io.bytes() > bem::kWsKeep) c->ip_io.release();
   return BEM_OK;
 }
 

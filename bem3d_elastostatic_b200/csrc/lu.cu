@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "lu.cuh"
+#include "tri_inv.cuh"
 
 namespace bem {
 
@@ -888,72 +889,26 @@ __global__ void trsm_small_kernel(T* S, int64_t lda, int k0, int w, int r_lo, in
     if (b < w) S[r + (int64_t)(k0 + b) * lda] = y[b];
 }
 
-// V = U^{-1} for the unit upper triangle U of S11 (jb x jb, jb <= 128); V column-major
-// (ldv).  Blocked by 32: four warps invert the diagonal blocks (lane j holds column j
-// of its block in registers and back-substitutes), then the off-diagonal blocks follow
-// in order of their distance from the diagonal,
-//   V_ij = -V_ii * sum_{k=i+1..j} U_ik V_kj,
-// each a 32 x 32 product spread over all 256 threads.  U is staged in shared memory,
-// V is written to (and re-read from) global memory by this CTA only.
-template <typename T>
-__global__ void __launch_bounds__(256) inv_unit_upper_kernel(const T* S11, int64_t lda, int jb, T* V, int ldv) {
+// V[b] = inverse of the unit upper triangle of diagonal block b of S11 (jb x jb, blocks of
+// 128), column-major with leading dimension 128; one CTA per block.
+__global__ void __launch_bounds__(kTriThreads) inv_unit_upper_f64_kernel(const double* S11, int64_t lda, int jb,
+                                                                         double* V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* U = reinterpret_cast<T*>(smem_raw);  // [128][128] column-major, zero outside the strict upper part
-  __shared__ T tmp[32 * 33];
-  constexpr int B = 32, NB = 128;
-  stage_block<T>(U, NB, S11, lda, jb, jb, NB, NB, [](int a, int b) { return a < b; });
-  __syncthreads();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nblk = (jb + B - 1) / B;
-  // diagonal blocks
-  if (warp < nblk) {
-    const int o = warp * B;
-    T x[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? T(1) : T(0);
-#pragma unroll
-    for (int i = B - 2; i >= 0; --i) {
-      T sacc = x[i];
-#pragma unroll
-      for (int k = i + 1; k < B; ++k) sacc -= U[(o + i) + (o + k) * NB] * x[k];
-      x[i] = (i < lane) ? sacc : x[i];
-    }
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-      if (o + i < jb && o + lane < jb) V[(o + i) + (int64_t)(o + lane) * ldv] = x[i];
-  }
-  // zero the strict lower blocks of V
-  for (int idx = tid; idx < jb * jb; idx += blockDim.x) {
-    const int r = idx % jb, cc = idx / jb;
-    if (r / B > cc / B) V[r + (int64_t)cc * ldv] = T(0);
-  }
-  __syncthreads();
-  for (int d = 1; d < nblk; ++d)
-    for (int bi = 0; bi + d < nblk; ++bi) {
-      const int bj = bi + d;
-      const int oi = bi * B, oj = bj * B;
-      // tmp = sum_{k=bi+1..bj} U_{bi,k} V_{k,bj}   (32 x 32)
-      for (int e = tid; e < B * B; e += blockDim.x) {
-        const int r = e % B, cc = e / B;
-        T acc = T(0);
-        for (int k = oi + B; k <= oj + B - 1 && k < jb; ++k) acc += U[(oi + r) + k * NB] * V[k + (int64_t)(oj + cc) * ldv];
-        tmp[r + cc * 33] = acc;
-      }
-      __syncthreads();
-      // V_{bi,bj} = -V_{bi,bi} tmp
-      for (int e = tid; e < B * B; e += blockDim.x) {
-        const int r = e % B, cc = e / B;
-        T acc = T(0);
-#pragma unroll 8
-        for (int k = 0; k < B; ++k) acc += V[(oi + r) + (int64_t)(oi + k) * ldv] * tmp[k + cc * 33];
-        if (oi + r < jb && oj + cc < jb) V[(oi + r) + (int64_t)(oj + cc) * ldv] = -acc;
-      }
-      __syncthreads();
-    }
+  double* U = reinterpret_cast<double*>(smem_raw);
+  const int o = kInvBlock * blockIdx.x, m = min(kInvBlock, jb - o);
+  stage_block<double>(U, kTriPitch, S11 + o + (int64_t)o * lda, lda, m, m, kInvBlock, kInvBlock,
+                      [](int a, int b) { return a < b; });
+  unit_upper_inverse(U, U + 128 * kTriPitch);
+  double* Vb = V + (size_t)blockIdx.x * kInvBlock * kInvBlock;
+  for (int idx = threadIdx.x; idx < kInvBlock * kInvBlock; idx += kTriThreads)
+    Vb[idx] = U[idx % kInvBlock + (idx / kInvBlock) * kTriPitch];
 }
 
-// The same inverse for FP32 factors with U and V both in shared memory (2 x 64 KB) and
-// the off-diagonal blocks of one distance from the diagonal computed together (two
+// The inverse of a unit upper triangle for FP32 factors with U and V both in shared memory
+// (2 x 64 KB), blocked by 32: four warps invert the diagonal blocks (lane j holds column j of
+// its block in registers and back-substitutes), then the off-diagonal blocks follow in order
+// of their distance from the diagonal, V_ij = -V_ii * sum_{k=i+1..j} U_ik V_kj, the
+// off-diagonal blocks of one distance from the diagonal computed together (two
 // barriers per distance); V is written to global memory once at the end.
 constexpr int kInvThreads = 512;
 
@@ -1269,6 +1224,8 @@ template int gemm<float>(bem_ctx*, int, int, int, const float*, int64_t, const f
 // ---------------------------------------------------------------------------------
 namespace {
 
+// FP64 sub-panels with as many lines as one cluster holds go to panel64.cu; wider ones and
+// the FP32 ones to the grid-synchronised panel_kernel.
 // The barrier counter grows monotonically over a factorisation (zeroed once with the
 // status words); each launch waits for its own arrivals on top of bar_base.
 template <typename T>
@@ -1276,6 +1233,8 @@ int panel_launch(bem_ctx* c, const LUWorkspace& ws, T* S, int64_t lda, int n, in
                  unsigned& bar_base) {
   static DeviceOnce checked;  // per instantiation (T) and device
   const int cols = n - r0;
+  if constexpr (sizeof(T) == 8)
+    if (cols <= panel_cluster_lines()) return panel_cluster_launch(c, S, lda, n, r0, w, piv, ws.status);
   static const int cap = [] {  // BEM_PANEL_CTAS: at most this many CTAs per panel launch
     const char* e = getenv("BEM_PANEL_CTAS");
     return e ? std::max(1, atoi(e)) : INT_MAX;
@@ -1394,9 +1353,11 @@ struct LUProfile {
 
 static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-// blocks of the TRSM-inverse region: FP32 factors keep the 2 x 4 inverses of a
-// window-pivoted 512-wide panel (panel_inv_f32_kernel), FP64 one block
-static size_t inv_blocks(int elem, int nb) { return elem == 4 ? 2 * (size_t)((nb + kInvBlock - 1) / kInvBlock) : 1; }
+// blocks of the TRSM-inverse region: FP32 factors keep both triangles' inverses of every
+// diagonal block of a panel (panel_inv_f32_kernel), FP64 the upper ones
+static size_t inv_blocks(int elem, int nb) {
+  return (elem == 4 ? 2 : 1) * (size_t)((nb + kInvBlock - 1) / kInvBlock);
+}
 
 static size_t finv_count(int elem, int nb) {
   return elem == 4 ? 2 * (size_t)nb * nb + 2 * (size_t)nb * kInvBlock : 0;
@@ -1475,8 +1436,8 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
   // window pivoting (pivot search within each sub-panel's diagonal block) or partial
   // pivoting (over every remaining row of T)
   const bool window = c->lu_window;
-  const size_t inv_smem = (size_t)kInvBlock * kInvBlock * sizeof(T);
-  cudaFuncSetAttribute(inv_unit_upper_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
+  const size_t inv_smem = kTriDoubles * sizeof(double);
+  cudaFuncSetAttribute(inv_unit_upper_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
   cudaFuncSetAttribute(inv_unit_upper_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)(2 * kInvBlock * kInvBlock * sizeof(float)));
   cudaFuncSetAttribute(panel_inv_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1670,21 +1631,25 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
       } else {
       // TRSM of the block row, Y = X U^{-1} with U the unit upper triangle of the panel's
       // diagonal block, in 128-wide column blocks: X_b -= Y_{<b} U_{<b,b}, Y_b = X_b inv(U_bb)
+      if constexpr (sizeof(T) == 8) {  // the inverses of the panel's diagonal blocks, in one launch
+        inv_unit_upper_f64_kernel<<<(jb + kInvBlock - 1) / kInvBlock, kTriThreads, inv_smem, c->stream>>>(
+            S + j0 + (int64_t)j0 * lda, lda, jb, V);
+        BEM_LAUNCH_CHECK(c);
+      }
       for (int b0 = 0; b0 < jb; b0 += kInvBlock) {
         const int bb = std::min(kInvBlock, jb - b0);
+        T* Vb = sizeof(T) == 8 ? V + (size_t)b0 * kInvBlock : V;
         T* Xb = S + t0 + (int64_t)(j0 + b0) * lda;
         if (b0 > 0 &&
             (rc = gemm<T>(c, m, bb, b0, Y, ldy, S + j0 + (int64_t)(j0 + b0) * lda, lda, Xb, lda, 0)))
           return rc;
-        if (sizeof(T) == 4)
+        if constexpr (sizeof(T) == 4) {
           inv_unit_upper_f32_kernel<<<1, kInvThreads, 2 * kInvBlock * kInvBlock * sizeof(float), c->stream>>>(
               reinterpret_cast<const float*>(S + (j0 + b0) + (int64_t)(j0 + b0) * lda), lda, bb,
               reinterpret_cast<float*>(V), kInvBlock);
-        else
-          inv_unit_upper_kernel<T><<<1, 256, inv_smem, c->stream>>>(
-              S + (j0 + b0) + (int64_t)(j0 + b0) * lda, lda, bb, V, kInvBlock);
-        BEM_LAUNCH_CHECK(c);
-        if ((rc = gemm<T>(c, m, bb, bb, Xb, lda, V, kInvBlock, Y + (int64_t)b0 * ldy, ldy, 1))) return rc;
+          BEM_LAUNCH_CHECK(c);
+        }
+        if ((rc = gemm<T>(c, m, bb, bb, Xb, lda, Vb, kInvBlock, Y + (int64_t)b0 * ldy, ldy, 1))) return rc;
       }
       }
       if (Yr == Y)
@@ -2017,98 +1982,53 @@ __global__ void permute_kernel(int n, const int* __restrict__ perm, const double
 // product, and the dependent chain per block is one publication, one tile product
 // (its loads issued before the wait) and one inverse product.
 
-constexpr int kInvPitch = kSolveBlock + 1;  // shared-memory pitch of the staged triangle
-
 // Dinv[2 blk] = inverse of the lower triangle (diagonal included) of the diagonal block
 // blk of S, Dinv[2 blk + 1] = inverse of its strict upper triangle plus the identity;
 // each 128 x 128, column-major, FP64, zero outside the block's order.  Both are the
-// inverse W of a unit upper triangle, blocked by 32 (the 32 x 32 diagonal blocks by
-// back substitution in registers, then W_ij = -W_ii sum_{k=i+1..j} U_ik W_kj by
-// distance from the diagonal): the upper one directly; for the lower one,
-// D = N diag(D) with N unit lower, so D^{-1} = diag(D)^{-1} N^{-1} and N^{-1} = W^T
-// for W = (N^T)^{-1}.  Grid (blocks, 2), blockIdx.y = 0 lower, 1 upper.
+// inverse W of a unit upper triangle (unit_upper_inverse): the upper one directly; for the
+// lower one, D = N diag(D) with N unit lower, so D^{-1} = diag(D)^{-1} N^{-1} and N^{-1} =
+// W^T for W = (N^T)^{-1}.  Grid (blocks, 2), blockIdx.y = 0 lower, 1 upper.
 template <typename T>
-__global__ void __launch_bounds__(256) diag_inv_kernel(const T* __restrict__ S, int64_t lda, int n,
-                                                       double* __restrict__ Dinv) {
+__global__ void __launch_bounds__(kTriThreads) diag_inv_kernel(const T* __restrict__ S, int64_t lda, int n,
+                                                               double* __restrict__ Dinv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* U = reinterpret_cast<double*>(smem_raw);  // [128][kInvPitch], the strict upper part
+  double* U = reinterpret_cast<double*>(smem_raw);  // [128][kTriPitch], the strict upper part
   __shared__ double dg[kSolveBlock];
-  __shared__ double tmp[32 * 33];
-  constexpr int B = 32, NB = kSolveBlock, P = kInvPitch;
+  constexpr int NB = kSolveBlock, P = kTriPitch;
   const int blk = blockIdx.x;
   const bool lower = blockIdx.y == 0;
   const int k0 = blk * NB, jb = min(NB, n - k0);
   const T* D = S + k0 + (int64_t)k0 * lda;
   double* V = Dinv + ((size_t)blk * 2 + blockIdx.y) * (NB * NB);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   if (tid < NB) dg[tid] = (tid < jb) ? (double)D[tid + (int64_t)tid * lda] : 1.0;
   __syncthreads();
   // U(a, b), a < b: S(a, b) for the upper inverse, S(b, a) / S(a, a) for the lower one;
-  // the index runs along S's columns (contiguous) in both cases
-  for (int idx = tid; idx < NB * NB; idx += blockDim.x) {
-    const int i = idx % NB, j = idx / NB;  // S(k0 + i, k0 + j)
-    const double v = (i < jb && j < jb) ? (double)D[i + (int64_t)j * lda] : 0.0;
-    if (lower) {
-      if (j < i) U[j + i * P] = v / dg[j];
-      else U[j + i * P] = 0.0;
-    } else {
-      U[i + j * P] = (i < j) ? v : 0.0;
+  // the index runs along S's columns (contiguous) in both cases, 16 loads in flight
+  for (int base = tid; base < NB * NB; base += 16 * kTriThreads) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = (base + u * kTriThreads) % NB, j = (base + u * kTriThreads) / NB;  // S(k0 + i, k0 + j)
+      v[u] = (i < jb && j < jb && (lower ? j < i : i < j)) ? (double)D[i + (int64_t)j * lda] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = (base + u * kTriThreads) % NB, j = (base + u * kTriThreads) / NB;
+      if (lower) U[j + i * P] = j < i ? v[u] / dg[j] : 0.0;
+      else U[i + j * P] = v[u];
     }
   }
-  __syncthreads();
-  const int nb32 = (jb + B - 1) / B;
-  if (warp < nb32) {
-    const int o = warp * B;
-    double x[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? 1.0 : 0.0;
-#pragma unroll
-    for (int i = B - 2; i >= 0; --i) {
-      double s = x[i];
-#pragma unroll
-      for (int k = i + 1; k < B; ++k) s = fma(-U[(o + i) + (o + k) * P], x[k], s);
-      x[i] = (i < lane) ? s : x[i];
+  unit_upper_inverse(U, U + 128 * P);
+  // the upper inverse, or diag(D)^{-1} W^T
+  for (int idx = tid; idx < NB * NB; idx += kTriThreads) {
+    const int i = idx % NB, j = idx / NB;
+    double v = 0.0;
+    if (i < jb && j < jb) {
+      if (!lower) v = U[i + j * P];
+      else if (j <= i) v = U[j + i * P] / dg[i];
     }
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-      if (o + i < jb && o + lane < jb) V[(o + i) + (o + lane) * NB] = x[i];
-  }
-  for (int idx = tid; idx < NB * NB; idx += blockDim.x) {
-    const int r = idx % NB, cc = idx / NB;
-    if (r >= jb || cc >= jb || r / B > cc / B) V[idx] = 0.0;
-  }
-  __syncthreads();
-  for (int d = 1; d < nb32; ++d)
-    for (int bi = 0; bi + d < nb32; ++bi) {
-      const int oi = bi * B, oj = (bi + d) * B;
-      for (int e = tid; e < B * B; e += blockDim.x) {
-        const int r = e % B, cc = e / B;
-        double acc = 0.0;
-        for (int k = oi + B; k < oj + B && k < jb; ++k) acc = fma(U[(oi + r) + k * P], V[k + (oj + cc) * NB], acc);
-        tmp[r + cc * 33] = acc;
-      }
-      __syncthreads();
-      for (int e = tid; e < B * B; e += blockDim.x) {
-        const int r = e % B, cc = e / B;
-        double acc = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < B; ++k) acc = fma(V[(oi + r) + (oi + k) * NB], tmp[k + cc * 33], acc);
-        if (oi + r < jb && oj + cc < jb) V[(oi + r) + (oj + cc) * NB] = -acc;
-      }
-      __syncthreads();
-    }
-  if (lower) {
-    // V := diag(D)^{-1} W^T, pairwise in place
-    for (int idx = tid; idx < NB * NB; idx += blockDim.x) {
-      const int i = idx % NB, j = idx / NB;
-      if (i < j) {
-        const double wij = V[i + j * NB], wji = V[j + i * NB];
-        V[i + j * NB] = wji / dg[i];
-        V[j + i * NB] = wij / dg[j];
-      } else if (i == j) {
-        V[i + i * NB] = (i < jb) ? 1.0 / dg[i] : 0.0;
-      }
-    }
+    V[idx] = v;
   }
 }
 
@@ -2514,13 +2434,13 @@ int lu_prepare_inverses(bem_ctx* c, const T* S, int64_t lda, int n) {
     c->dinv.release();
     BEM_CUDA(c, c->dinv.alloc(need));
   }
-  const int smem = kSolveBlock * kInvPitch * (int)sizeof(double);
+  const int smem = kTriDoubles * (int)sizeof(double);
   static DeviceOnce attr;  // per instantiation and device
   if (attr.pending()) {
     BEM_CUDA(c, cudaFuncSetAttribute(diag_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr.mark();
   }
-  diag_inv_kernel<T><<<dim3(nblk, 2), 256, smem, c->stream>>>(S, lda, n, c->dinv.p);
+  diag_inv_kernel<T><<<dim3(nblk, 2), kTriThreads, smem, c->stream>>>(S, lda, n, c->dinv.p);
   BEM_LAUNCH_CHECK(c);
   c->dinv_src = S;
   c->dinv_n = n;

@@ -11,13 +11,11 @@
 //               assembly_mod.f90:125-218 (A(:, dof) = H(:, dof) unless u is known there,
 //               minus mu G for every element that prescribes u at that node), then
 //               the pinned rows
-//   solve       a persistent kernel factors one system per CTA (LAPACK dgetrf: row
-//               pivoting of A, 32-wide panels, SMEM-staged 64 x 64 trailing tiles), in
-//               FP32 (refined) or FP64 (plain); the substitution for all load cases
-//               and the FP64 residual / backward error of each system follow, one CTA
-//               per system, for a fixed number of refinement sweeps in which converged
-//               systems skip their work.  The whole solve is captured once in a CUDA
-//               graph and replayed.
+//   solve       batch_lu.cu: the LU of all systems panel by panel (LAPACK dgetrf: row
+//               pivoting of A), in FP32 (refined) or FP64 (plain), then the substitution
+//               for all load cases and the FP64 residual / backward error of each system,
+//               for a fixed number of refinement sweeps in which converged systems skip
+//               their work.  The whole solve is captured once in a CUDA graph and replayed.
 //
 // The column swap is formed from H and G, so a node's prescribed displacement must be
 // the same in every element that prescribes it (the single-system path takes each
@@ -31,30 +29,11 @@
 #include <vector>
 
 #include "asm_args.cuh"
+#include "batch_dev.cuh"
 #include "common.cuh"
 
 namespace bem {
 namespace {
-
-constexpr int kLuNB = 32;              // panel width of the per-system LU
-constexpr int kTM = 128, kTN = 64;     // trailing-update tile (kTM x kTN)
-constexpr int kMaxRhs = 8;             // load cases per system
-constexpr int kSolveThreads = 512;
-constexpr size_t kSolveSmem = 200 * 1024;  // substitution workspace per CTA
-
-struct SysDev {
-  int n, ne, N, nrhs;
-  int64_t lda;   // of H / A and of the factor copy
-  int64_t ldg;   // of G
-  int64_t a_off, g_off, f_off;  // A (FP64), G (FP64), factor (T) in their arenas
-  int64_t v_off;                // FI, X, R: N x nrhs each (ld N) in the vector arena
-  int64_t piv_off;
-  int64_t cs_off, ncs;          // column-swap list: (dof, G column) pairs
-  int64_t fl_off, nfl;          // FI terms: (matrix, column) and nrhs coefficients each
-  int64_t pin_off, npins;
-  int64_t uk_off;               // u known per dof
-  double mu;
-};
 
 // ---------------------------------------------------------------------------------
 // combine
@@ -112,470 +91,6 @@ __global__ void batch_pins_kernel(const SysDev* __restrict__ sys, const int* __r
   if (threadIdx.x < S.nrhs) FI[S.v_off + p + (int64_t)threadIdx.x * S.N] = 0.0;
 }
 
-// ---------------------------------------------------------------------------------
-// per-system LU (one CTA), substitution and residual
-// ---------------------------------------------------------------------------------
-
-template <typename T>
-__global__ void batch_copy_kernel(const SysDev* __restrict__ sys, const double* __restrict__ A,
-                                  T* __restrict__ F) {
-  const SysDev S = sys[blockIdx.y];
-  const int64_t total = (int64_t)S.N * S.lda;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x)
-    F[S.f_off + k] = (T)A[S.a_off + k];
-}
-
-__device__ __forceinline__ void take_max(double& bv, int& bi, double v, int i) {
-  if (v > bv || (v == bv && i < bi)) {
-    bv = v;
-    bi = i;
-  }
-}
-
-// dynamic shared memory of the LU kernel: the L21 (kLuNB x kTM) and U12 (kLuNB x kTN) tiles
-template <typename T>
-constexpr size_t lu_smem() { return (size_t)kLuNB * (kTM + kTN) * sizeof(T); }
-
-template <typename T, int NT>
-__device__ void cta_getrf(T* A, int64_t lda, int N, int* ipiv, int* info, T* s_a, T* s_b) {
-  __shared__ double s_v[NT / 32];
-  __shared__ int s_i[NT / 32];
-  __shared__ int s_piv[kLuNB];
-  __shared__ int s_rows[2 * kLuNB], s_src[2 * kLuNB], s_nrows;
-  __shared__ T s_row[kLuNB];
-  __shared__ T s_L[kLuNB][kLuNB + 1];
-  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-  if (tid == 0) *info = 0;
-  for (int j0 = 0; j0 < N; j0 += kLuNB) {
-    const int jb = min(kLuNB, N - j0);
-    // ---- panel: columns j0 .. j0+jb-1 ------------------------------------------------
-    for (int j = j0; j < j0 + jb; ++j) {
-      double bv = -1.0;
-      int bi = INT_MAX;
-      for (int i = j + tid; i < N; i += NT) take_max(bv, bi, fabs((double)A[i + (int64_t)j * lda]), i);
-      for (int off = 16; off > 0; off >>= 1) {
-        const double ov = __shfl_xor_sync(0xffffffffu, bv, off);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-        take_max(bv, bi, ov, oi);
-      }
-      if (lane == 0) {
-        s_v[wp] = bv;
-        s_i[wp] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        for (int w = 1; w < NT / 32; ++w) take_max(bv, bi, s_v[w], s_i[w]);
-        s_piv[j - j0] = bi;
-        ipiv[j] = bi;
-        if (bv == 0.0 && *info == 0) *info = j + 1;
-      }
-      __syncthreads();
-      const int p = s_piv[j - j0];
-      if (p != j && tid < jb) {
-        T* a = A + j + (int64_t)(j0 + tid) * lda;
-        T* b = A + p + (int64_t)(j0 + tid) * lda;
-        const T t = *a;
-        *a = *b;
-        *b = t;
-      }
-      __syncthreads();
-      const T piv = A[j + (int64_t)j * lda];
-      if (tid < jb) s_row[tid] = A[j + (int64_t)(j0 + tid) * lda];
-      __syncthreads();
-      if (piv != T(0)) {
-        for (int i = j + 1 + tid; i < N; i += NT) {
-          T* ri = A + i;
-          const T l = ri[(int64_t)j * lda] / piv;
-          ri[(int64_t)j * lda] = l;
-          for (int c = j + 1 - j0; c < jb; ++c) ri[(int64_t)(j0 + c) * lda] -= l * s_row[c];
-        }
-      }
-      __syncthreads();
-    }
-    // ---- the panel's interchanges on the other columns, as one gather per column ---
-    if (tid == 0) {
-      int nr = 0;
-      for (int q = 0; q < jb; ++q) {  // rows touched: j0+q and their pivots
-        const int cand[2] = {j0 + q, s_piv[q]};
-        for (int u = 0; u < 2; ++u) {
-          int f = -1;
-          for (int m = 0; m < nr; ++m)
-            if (s_rows[m] == cand[u]) f = m;
-          if (f < 0) {
-            s_rows[nr] = cand[u];
-            s_src[nr] = cand[u];
-            ++nr;
-          }
-        }
-      }
-      for (int q = 0; q < jb; ++q) {  // apply the swaps to the labels in order
-        int a = -1, b = -1;
-        for (int m = 0; m < nr; ++m) {
-          if (s_rows[m] == j0 + q) a = m;
-          if (s_rows[m] == s_piv[q]) b = m;
-        }
-        const int t = s_src[a];
-        s_src[a] = s_src[b];
-        s_src[b] = t;
-      }
-      s_nrows = nr;
-    }
-    __syncthreads();
-    {
-      const int nr = s_nrows;
-      for (int c = wp; c < N; c += NT / 32) {
-        if (c >= j0 && c < j0 + jb) continue;
-        T* col = A + (int64_t)c * lda;
-        T v0 = T(0), v1 = T(0);
-        if (lane < nr) v0 = col[s_src[lane]];
-        if (lane + 32 < nr) v1 = col[s_src[lane + 32]];
-        __syncwarp();
-        if (lane < nr) col[s_rows[lane]] = v0;
-        if (lane + 32 < nr) col[s_rows[lane + 32]] = v1;
-      }
-    }
-    __syncthreads();
-    const int t0 = j0 + jb;
-    if (t0 >= N) break;
-    // ---- U12 = L11^{-1} A12 (unit lower), one column per thread -------------------
-    for (int idx = tid; idx < jb * jb; idx += NT) {
-      const int r = idx % jb, c = idx / jb;
-      s_L[r][c] = A[j0 + r + (int64_t)(j0 + c) * lda];
-    }
-    __syncthreads();
-    for (int c = t0 + tid; c < N; c += NT) {
-      T* col = A + j0 + (int64_t)c * lda;
-      T x[kLuNB];
-#pragma unroll
-      for (int q = 0; q < kLuNB; ++q) {
-        if (q < jb) {
-          T v = col[q];
-#pragma unroll
-          for (int t = 0; t < q; ++t) v -= s_L[q][t] * x[t];
-          x[q] = v;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kLuNB; ++q)
-        if (q < jb) col[q] = x[q];
-    }
-    __syncthreads();
-    // ---- A22 -= L21 U12, tiles of kTM x kTN: the tile of C is loaded with the operand
-    //      tiles, so a tile costs one memory round trip before its FMAs ---------------
-    const int m = N - t0;
-    const int tm = (m + kTM - 1) / kTM, tn = (m + kTN - 1) / kTN;
-    constexpr int CPT = kTM * kTN / NT;  // columns per thread
-    const int r = tid % kTM, cg = tid / kTM;
-    for (int tt = 0; tt < tm * tn; ++tt) {
-      const int ti = tt % tm, tj = tt / tm;
-      const int rb = t0 + ti * kTM, cb = t0 + tj * kTN;
-      for (int idx = tid; idx < kLuNB * kTM; idx += NT) {
-        const int rr = idx % kTM, k = idx / kTM;  // L21(rb + rr, j0 + k)
-        s_a[k * kTM + rr] = (k < jb && rb + rr < N) ? A[rb + rr + (int64_t)(j0 + k) * lda] : T(0);
-      }
-      for (int idx = tid; idx < kLuNB * kTN; idx += NT) {
-        const int kk = idx % kLuNB, cc = idx / kLuNB;  // U12(j0 + kk, cb + cc)
-        s_b[kk * kTN + cc] = (kk < jb && cb + cc < N) ? A[j0 + kk + (int64_t)(cb + cc) * lda] : T(0);
-      }
-      T acc[CPT];
-      const bool row_ok = rb + r < N;
-#pragma unroll
-      for (int q = 0; q < CPT; ++q) {
-        const int cc = cb + cg * CPT + q;
-        acc[q] = (row_ok && cc < N) ? A[rb + r + (int64_t)cc * lda] : T(0);
-      }
-      __syncthreads();
-#pragma unroll 4
-      for (int k = 0; k < kLuNB; ++k) {
-        const T l = s_a[k * kTM + r];
-#pragma unroll
-        for (int q = 0; q < CPT; ++q) acc[q] = fma(-l, s_b[k * kTN + cg * CPT + q], acc[q]);
-      }
-      if (row_ok) {
-#pragma unroll
-        for (int q = 0; q < CPT; ++q) {
-          const int cc = cb + cg * CPT + q;
-          if (cc < N) A[rb + r + (int64_t)cc * lda] = acc[q];
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-template <typename T, int NT>
-__global__ void __launch_bounds__(NT) batch_lu_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order,
-                                                      int nsys, T* F, int* piv, int* info, unsigned* counter) {
-  extern __shared__ __align__(16) unsigned char lu_dyn[];
-  T* s_a = reinterpret_cast<T*>(lu_dyn);
-  T* s_b = s_a + kLuNB * kTM;
-  __shared__ int s_item;
-  for (;;) {
-    if (threadIdx.x == 0) s_item = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    const int it = s_item;
-    __syncthreads();
-    if (it >= nsys) return;
-    const int s = order[it];
-    const SysDev S = sys[s];
-    cta_getrf<T, NT>(F + S.f_off, S.lda, S.N, piv + S.piv_off, info + s, s_a, s_b);
-    __syncthreads();
-  }
-}
-
-// X (+)= U^{-1} L^{-1} P^T R for the system's load cases, in shared memory chunks of
-// nc columns (B is [N][nc]); converged systems are skipped
-template <typename T>
-__global__ void __launch_bounds__(kSolveThreads)
-    batch_solve_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order, int nsys,
-                       const T* __restrict__ F, const int* __restrict__ piv, const double* __restrict__ R,
-                       double* __restrict__ X, const int* __restrict__ conv, const int* __restrict__ info,
-                       int accumulate, unsigned* counter) {
-  extern __shared__ double sB[];
-  __shared__ int s_item;
-  __shared__ double s_x[kLuNB][kMaxRhs];
-  __shared__ double s_d[kLuNB][kLuNB + 1];
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (;;) {
-    if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    const int it = s_item;
-    __syncthreads();
-    if (it >= nsys) return;
-    const int s = order[it];
-    if (conv[s] || info[s]) continue;  // converged, or a zero pivot
-    const SysDev S = sys[s];
-    const int N = S.N;
-    const T* A = F + S.f_off;
-    const int* pv = piv + S.piv_off;
-    const int nc_max = max(1, min(S.nrhs, (int)(kSolveSmem / (sizeof(double) * (size_t)N))));
-    for (int r0 = 0; r0 < S.nrhs; r0 += nc_max) {
-      const int nc = min(nc_max, S.nrhs - r0);
-      for (int i = tid; i < N; i += kSolveThreads)
-        _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) sB[i * nc + r] = R[S.v_off + i + (int64_t)(r0 + r) * N];
-      __syncthreads();
-      if (tid < nc)
-        for (int j = 0; j < N; ++j) {
-          const int p = pv[j];
-          if (p != j) {
-            const double t = sB[j * nc + tid];
-            sB[j * nc + tid] = sB[p * nc + tid];
-            sB[p * nc + tid] = t;
-          }
-        }
-      __syncthreads();
-      // forward, unit lower, blocks of 32
-      for (int j0 = 0; j0 < N; j0 += kLuNB) {
-        const int jb = min(kLuNB, N - j0);
-        for (int idx = tid; idx < kLuNB * kLuNB; idx += kSolveThreads) {  // the diagonal block
-          const int rr = idx % kLuNB, cc = idx / kLuNB;
-          s_d[rr][cc] = (rr < jb && cc < jb) ? (double)A[j0 + rr + (int64_t)(j0 + cc) * S.lda] : 0.0;
-        }
-        __syncthreads();
-        if (tid < 32) {
-          double b[kMaxRhs];
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) b[r] = (lane < jb) ? sB[(j0 + lane) * nc + r] : 0.0;
-          for (int t = 0; t < jb; ++t) {
-            const double l = (lane > t && lane < jb) ? s_d[lane][t] : 0.0;
-            _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) {
-              const double xt = __shfl_sync(0xffffffffu, b[r], t);
-              b[r] = fma(-l, xt, b[r]);
-            }
-          }
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc)
-            if (lane < jb) {
-              sB[(j0 + lane) * nc + r] = b[r];
-              s_x[lane][r] = b[r];
-            }
-        }
-        __syncthreads();
-        for (int i = j0 + jb + tid; i < N; i += kSolveThreads) {
-          double acc[kMaxRhs];
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) acc[r] = sB[i * nc + r];
-          for (int q0 = 0; q0 < jb; q0 += 8) {  // eight loads in flight, then their FMAs
-            T lv[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) lv[u] = (q0 + u < jb) ? A[i + (int64_t)(j0 + q0 + u) * S.lda] : T(0);
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const double l = (double)lv[u];
-              _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) acc[r] = fma(-l, s_x[q0 + u < jb ? q0 + u : 0][r], acc[r]);
-            }
-          }
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) sB[i * nc + r] = acc[r];
-        }
-        __syncthreads();
-      }
-      // backward, non-unit upper, blocks of 32 from the last
-      for (int j0 = ((N - 1) / kLuNB) * kLuNB; j0 >= 0; j0 -= kLuNB) {
-        const int jb = min(kLuNB, N - j0);
-        for (int idx = tid; idx < kLuNB * kLuNB; idx += kSolveThreads) {
-          const int rr = idx % kLuNB, cc = idx / kLuNB;
-          s_d[rr][cc] = (rr < jb && cc < jb) ? (double)A[j0 + rr + (int64_t)(j0 + cc) * S.lda] : 0.0;
-        }
-        __syncthreads();
-        if (tid < 32) {
-          double b[kMaxRhs];
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) b[r] = (lane < jb) ? sB[(j0 + lane) * nc + r] : 0.0;
-          for (int t = jb - 1; t >= 0; --t) {
-            const double d = s_d[t][t];
-            const double u = (lane < t) ? s_d[lane][t] : 0.0;
-            _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) {
-              const double xt = __shfl_sync(0xffffffffu, b[r], t) / d;
-              if (lane == t) b[r] = xt;
-              else b[r] = fma(-u, xt, b[r]);
-            }
-          }
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc)
-            if (lane < jb) {
-              sB[(j0 + lane) * nc + r] = b[r];
-              s_x[lane][r] = b[r];
-            }
-        }
-        __syncthreads();
-        for (int i = tid; i < j0; i += kSolveThreads) {
-          double acc[kMaxRhs];
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) acc[r] = sB[i * nc + r];
-          for (int q0 = 0; q0 < jb; q0 += 8) {  // eight loads in flight, then their FMAs
-            T uv[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) uv[k] = (q0 + k < jb) ? A[i + (int64_t)(j0 + q0 + k) * S.lda] : T(0);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              const double u = (double)uv[k];
-              _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) acc[r] = fma(-u, s_x[q0 + k < jb ? q0 + k : 0][r], acc[r]);
-            }
-          }
-          _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) sB[i * nc + r] = acc[r];
-        }
-        __syncthreads();
-      }
-      for (int i = tid; i < N; i += kSolveThreads)
-        _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nc) {
-          double* xo = X + S.v_off + i + (int64_t)(r0 + r) * N;
-          *xo = accumulate ? *xo + sB[i * nc + r] : sB[i * nc + r];
-        }
-      __syncthreads();
-    }
-  }
-}
-
-// R = B - A X (FP64) and the backward error max_r ||R_r|| / (||A|| ||X_r|| + ||B_r||)
-// (infinity norms); conv[s] = 1 once it is <= tol, 2 once a sweep gains less than 10 %
-__global__ void __launch_bounds__(kSolveThreads)
-    batch_residual_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order, int nsys,
-                          const double* __restrict__ A, const double* __restrict__ B, const double* __restrict__ X,
-                          double* __restrict__ R, double* __restrict__ berr, int* __restrict__ conv,
-                          const int* __restrict__ info, double tol, int first, unsigned* counter) {
-  extern __shared__ double sX[];
-  __shared__ int s_item;
-  __shared__ double s_red[kSolveThreads / 32][3 * kMaxRhs + 1];
-  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-  for (;;) {
-    if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    const int it = s_item;
-    __syncthreads();
-    if (it >= nsys) return;
-    const int s = order[it];
-    if (conv[s] || info[s]) continue;
-    const SysDev S = sys[s];
-    const int N = S.N, nrhs = S.nrhs;
-    const double* As = A + S.a_off;
-    // X staged in chunks of columns; the row loop keeps all nrhs partial sums
-    double rmax[kMaxRhs], xmax[kMaxRhs], bmax[kMaxRhs], amax = 0.0;
-    for (int r = 0; r < kMaxRhs; ++r) rmax[r] = xmax[r] = bmax[r] = 0.0;
-    const int rows_per = (N + kSolveThreads - 1) / kSolveThreads;
-    for (int rb = 0; rb < rows_per; ++rb) {
-      const int i = tid + rb * kSolveThreads;
-      double acc[kMaxRhs], asum = 0.0;
-      _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) acc[r] = (i < N) ? B[S.v_off + i + (int64_t)r * N] : 0.0;
-      const int ncol = max(1, (int)(kSolveSmem / (sizeof(double) * (size_t)nrhs)));
-      for (int c0 = 0; c0 < N; c0 += ncol) {
-        const int cn = min(ncol, N - c0);
-        __syncthreads();
-        for (int k = tid; k < cn * nrhs; k += kSolveThreads) {
-          const int c = k % cn, r = k / cn;
-          sX[c * nrhs + r] = X[S.v_off + c0 + c + (int64_t)r * N];
-        }
-        __syncthreads();
-        if (i < N) {
-          // eight columns per step: eight independent loads in flight per thread (one
-          // CTA per system streams its whole A, so memory-level parallelism sets the time)
-          int c = 0;
-          for (; c + 8 <= cn; c += 8) {
-            double a[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = As[i + (int64_t)(c0 + c + u) * S.lda];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              asum += fabs(a[u]);
-              _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) acc[r] = fma(-a[u], sX[(c + u) * nrhs + r], acc[r]);
-            }
-          }
-          for (; c < cn; ++c) {
-            const double a = As[i + (int64_t)(c0 + c) * S.lda];
-            asum += fabs(a);
-            _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) acc[r] = fma(-a, sX[c * nrhs + r], acc[r]);
-          }
-        }
-      }
-      if (i < N) {
-        amax = fmax(amax, asum);
-        _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) {
-          R[S.v_off + i + (int64_t)r * N] = acc[r];
-          rmax[r] = fmax(rmax[r], fabs(acc[r]));
-          xmax[r] = fmax(xmax[r], fabs(X[S.v_off + i + (int64_t)r * N]));
-          bmax[r] = fmax(bmax[r], fabs(B[S.v_off + i + (int64_t)r * N]));
-        }
-      }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-      amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-      _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) {
-        rmax[r] = fmax(rmax[r], __shfl_xor_sync(0xffffffffu, rmax[r], off));
-        xmax[r] = fmax(xmax[r], __shfl_xor_sync(0xffffffffu, xmax[r], off));
-        bmax[r] = fmax(bmax[r], __shfl_xor_sync(0xffffffffu, bmax[r], off));
-      }
-    }
-    if (lane == 0) {
-      _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) {
-        s_red[wp][r] = rmax[r];
-        s_red[wp][kMaxRhs + r] = xmax[r];
-        s_red[wp][2 * kMaxRhs + r] = bmax[r];
-      }
-      s_red[wp][3 * kMaxRhs] = amax;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      double an = 0.0, be = 0.0;
-      for (int w = 0; w < kSolveThreads / 32; ++w) an = fmax(an, s_red[w][3 * kMaxRhs]);
-      _Pragma("unroll") for (int r = 0; r < kMaxRhs; ++r) if (r < nrhs) {
-        double rn = 0.0, xn = 0.0, bn = 0.0;
-        for (int w = 0; w < kSolveThreads / 32; ++w) {
-          rn = fmax(rn, s_red[w][r]);
-          xn = fmax(xn, s_red[w][kMaxRhs + r]);
-          bn = fmax(bn, s_red[w][2 * kMaxRhs + r]);
-        }
-        const double den = an * xn + bn;
-        be = fmax(be, den > 0.0 ? rn / den : 0.0);
-      }
-      const double prev = berr[s];
-      berr[s] = be;
-      if (!first) {
-        if (be <= tol) conv[s] = 1;
-        else if (be > 0.9 * prev) conv[s] = 2;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void zero_kernel(double* p, int64_t n) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = 0.0;
-}
-
 }  // namespace
 }  // namespace bem
 
@@ -603,6 +118,9 @@ struct bem_batch {
   int factored_precision = -1;
   // device storage
   bem::DBuf<double> x, y, z, ref, tab, H, G, vec, berr, A64f;
+  bem::DBuf<double> W, dinv, red;  // solve: the sweeps' vectors, diagonal-block inverses, maxima
+  bem::DBuf<int> perm, moved, lu_err;
+  int64_t rows = 0, inv_blocks = 0;  // of all systems
   bem::DBuf<float> A32;
   bem::DBuf<int> nconec, kconec_loc, kconec_glob, nesim, ke, batches, node_off, piv, info, conv, uk_csr, ord;
   bem::DBuf<int2> tiles, cs, terms;
@@ -616,8 +134,8 @@ struct bem_batch {
   cudaGraphExec_t graph = nullptr;
   int graph_key[3] = {-1, -1, -1};
   double graph_tol = -1.0;
-  int lu_threads = 0;  // autotuned per batch: 256 or 512
-  float lu_ms[2] = {0.f, 0.f};
+  long long graph_launches = 0;
+  int lu_threads = 0;  // CTA size of the LU the solve took
   ~bem_batch() {
     if (graph) cudaGraphExecDestroy(graph);
     if (stream) cudaStreamDestroy(stream);
@@ -731,6 +249,10 @@ int bem_batch_add(bem_batch* b, int n, int ne, const double* x, const double* y,
     if (pins[i] < 0 || pins[i] >= 3 * n) return bfail(b, BEM_ERR_ARG, "batch_add: pin out of range");
   b->sys.push_back(std::move(s));
   b->assembled = b->factored = false;
+  if (b->graph) {  // captured for the systems so far
+    cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+  }
   return (int)b->sys.size() - 1;
 }
 
@@ -745,7 +267,7 @@ int bem_batch_assemble(bem_batch* b) {
   std::vector<double> hcoef;
   std::vector<int> huk;  // per system: N u-known flags, then N + 1 row pointers of the cs list
   std::vector<bem::SysDev> hs(ns);
-  int64_t a_off = 0, g_off = 0, v_off = 0, piv_off = 0, elem_off = 0, batch_off = 0;
+  int64_t a_off = 0, g_off = 0, v_off = 0, piv_off = 0, inv_off = 0, elem_off = 0, batch_off = 0;
   std::vector<int64_t> elem_offs(ns), batch_offs(ns), node_offs(ns);
   std::vector<int> nbatches(ns);
   for (int si = 0; si < ns; ++si) {
@@ -767,6 +289,8 @@ int bem_batch_assemble(bem_batch* b) {
     v_off += (int64_t)N * nrhs;
     D.piv_off = piv_off;
     piv_off += N;
+    D.inv_off = inv_off;
+    inv_off += (N + 127) / 128;
     D.mu = S.mu;
     node_offs[si] = hx.size();
     hnode_off[si] = (int)hx.size();
@@ -920,6 +444,8 @@ int bem_batch_assemble(bem_batch* b) {
   BB_CUDA(b, b->conv.alloc(ns));
   BB_CUDA(b, b->berr.alloc(ns));
   BB_CUDA(b, b->counters.alloc(64));
+  b->rows = piv_off;
+  b->inv_blocks = inv_off;
   // per-system assembly arguments (mode HG)
   std::vector<bem::AsmArgs> hargs(ns);
   for (int si = 0; si < ns; ++si) {
@@ -979,99 +505,6 @@ int bem_batch_assemble(bem_batch* b) {
 
 // bem_batch_info: include/bem3d_b200.h
 
-namespace {
-
-template <typename T, int NT>
-int launch_lu(bem_batch* b, T* F) {
-  static bem::DeviceOnce attr;
-  if (attr.pending()) {
-    if (cudaFuncSetAttribute(bem::batch_lu_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)bem::lu_smem<T>()) != cudaSuccess)
-      return BEM_ERR_CUDA;
-    attr.mark();
-  }
-  bem::batch_lu_kernel<T, NT><<<std::min((int)b->sys.size(), b->sm_count), NT, bem::lu_smem<T>(), b->stream>>>(
-      b->dsys.p, b->ord.p, (int)b->sys.size(), F, b->piv.p, b->info.p, b->counters.p + 0);
-  return cudaGetLastError() == cudaSuccess ? BEM_OK : BEM_ERR_CUDA;
-}
-
-template <typename T>
-int enqueue_solve(bem_batch* b, int precision, double tol, int sweeps, T* F) {
-  const int ns = (int)b->sys.size();
-  const int64_t nv = b->vec.count / 3;
-  double *FI = b->vec.p, *X = b->vec.p + nv, *R = b->vec.p + 2 * nv;
-  const int grid = std::min(ns, b->sm_count);
-  BB_CUDA(b, cudaMemsetAsync(b->counters.p, 0, b->counters.bytes(), b->stream));
-  BB_CUDA(b, cudaMemsetAsync(b->conv.p, 0, b->conv.bytes(), b->stream));
-  bem::batch_copy_kernel<T><<<dim3(64, ns), 256, 0, b->stream>>>(b->dsys.p, b->H.p, F);
-  BB_CUDA(b, cudaGetLastError());
-  int rc = (b->lu_threads == 256) ? launch_lu<T, 256>(b, F) : launch_lu<T, 512>(b, F);
-  if (rc) return bfail(b, rc, "batch LU launch failed");
-  unsigned* cnt = b->counters.p + 1;
-  if (precision == BEM_PREC_FP64) {
-    bem::batch_solve_kernel<T><<<grid, bem::kSolveThreads, bem::kSolveSmem, b->stream>>>(
-        b->dsys.p, b->ord.p, ns, F, b->piv.p, FI, X, b->conv.p, b->info.p, 0, cnt++);
-    bem::batch_residual_kernel<<<grid, bem::kSolveThreads, bem::kSolveSmem, b->stream>>>(
-        b->dsys.p, b->ord.p, ns, b->H.p, FI, X, R, b->berr.p, b->conv.p, b->info.p, tol, 1, cnt++);
-  } else {
-    bem::zero_kernel<<<256, 256, 0, b->stream>>>(X, nv);
-    bem::batch_residual_kernel<<<grid, bem::kSolveThreads, bem::kSolveSmem, b->stream>>>(
-        b->dsys.p, b->ord.p, ns, b->H.p, FI, X, R, b->berr.p, b->conv.p, b->info.p, tol, 1, cnt++);
-    for (int it = 0; it < sweeps; ++it) {
-      bem::batch_solve_kernel<T><<<grid, bem::kSolveThreads, bem::kSolveSmem, b->stream>>>(
-          b->dsys.p, b->ord.p, ns, F, b->piv.p, R, X, b->conv.p, b->info.p, 1, cnt++);
-      bem::batch_residual_kernel<<<grid, bem::kSolveThreads, bem::kSolveSmem, b->stream>>>(
-          b->dsys.p, b->ord.p, ns, b->H.p, FI, X, R, b->berr.p, b->conv.p, b->info.p, tol, 0, cnt++);
-    }
-  }
-  BB_CUDA(b, cudaGetLastError());
-  return BEM_OK;
-}
-
-template <typename T>
-int set_smem() {
-  static bem::DeviceOnce done;
-  if (!done.pending()) return BEM_OK;
-  if (cudaFuncSetAttribute(bem::batch_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)bem::kSolveSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(bem::batch_residual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)bem::kSolveSmem) != cudaSuccess)
-    return BEM_ERR_CUDA;
-  done.mark();
-  return BEM_OK;
-}
-
-// the LU's CTA size: both candidates timed on this batch, the faster kept
-template <typename T>
-int autotune_lu(bem_batch* b, T* F) {
-  if (b->lu_threads) return BEM_OK;
-  const int ns = (int)b->sys.size();
-  cudaEvent_t e[3];
-  for (auto& x : e) BB_CUDA(b, cudaEventCreate(&x));
-  BB_CUDA(b, cudaMemsetAsync(b->counters.p, 0, sizeof(unsigned), b->stream));
-  bem::batch_copy_kernel<T><<<dim3(64, ns), 256, 0, b->stream>>>(b->dsys.p, b->H.p, F);
-  BB_CUDA(b, cudaEventRecord(e[0], b->stream));
-  if (launch_lu<T, 256>(b, F)) return bfail(b, BEM_ERR_CUDA, "batch LU launch failed");
-  BB_CUDA(b, cudaEventRecord(e[1], b->stream));
-  BB_CUDA(b, cudaMemsetAsync(b->counters.p, 0, sizeof(unsigned), b->stream));
-  bem::batch_copy_kernel<T><<<dim3(64, ns), 256, 0, b->stream>>>(b->dsys.p, b->H.p, F);
-  BB_CUDA(b, cudaEventRecord(e[2], b->stream));
-  if (launch_lu<T, 512>(b, F)) return bfail(b, BEM_ERR_CUDA, "batch LU launch failed");
-  cudaEvent_t e3;
-  BB_CUDA(b, cudaEventCreate(&e3));
-  BB_CUDA(b, cudaEventRecord(e3, b->stream));
-  BB_CUDA(b, cudaEventSynchronize(e3));
-  cudaEventElapsedTime(&b->lu_ms[0], e[0], e[1]);
-  cudaEventElapsedTime(&b->lu_ms[1], e[2], e3);
-  for (auto& x : e) cudaEventDestroy(x);
-  cudaEventDestroy(e3);
-  b->lu_threads = (b->lu_ms[0] <= b->lu_ms[1]) ? 256 : 512;
-  b->launches += 4;
-  return BEM_OK;
-}
-
-}  // namespace
-
 extern "C" {
 
 int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_batch_info* info) {
@@ -1080,30 +513,58 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
     return bfail(b, BEM_ERR_ARG, "batch_solve: precision must be BEM_PREC_FP64 or BEM_PREC_FP32_IR");
   if (max_iter < 1 || max_iter > 30) return bfail(b, BEM_ERR_ARG, "batch_solve: max_iter must be in 1..30");
   for (const auto& D : b->hdev)
-    if ((size_t)D.N * sizeof(double) > bem::kSolveSmem)
-      return bfail(b, BEM_ERR_TOO_LARGE, "batch_solve: a system of order above 25,600");
+    if (D.N > 25600) return bfail(b, BEM_ERR_TOO_LARGE, "batch_solve: a system of order above 25,600");
   BB_CUDA(b, cudaSetDevice(b->device));
   int rc;
   const int ns = (int)b->sys.size();
   const int sweeps = precision == BEM_PREC_FP64 ? 0 : max_iter;
   if (precision == BEM_PREC_FP64) {
-    if ((rc = set_smem<double>())) return bfail(b, rc, "batch_solve: shared memory attribute");
     if (b->A64f.count < b->H.count) BB_CUDA(b, b->A64f.alloc(b->H.count));
-    if ((rc = autotune_lu<double>(b, b->A64f.p))) return rc;
   } else {
-    if ((rc = set_smem<float>())) return bfail(b, rc, "batch_solve: shared memory attribute");
     if (b->A32.count < b->H.count) BB_CUDA(b, b->A32.alloc(b->H.count));
-    if ((rc = autotune_lu<float>(b, b->A32.p))) return rc;
   }
+  BB_CUDA(b, b->W.alloc((size_t)b->rows * bem::kMaxRhs));
+  BB_CUDA(b, b->dinv.alloc((size_t)b->inv_blocks * 2 * 128 * 128));
+  BB_CUDA(b, b->red.alloc((size_t)ns * (3 * bem::kMaxRhs + 1)));
+  BB_CUDA(b, b->perm.alloc((size_t)b->rows));
+  BB_CUDA(b, b->moved.alloc((size_t)ns * 64));
+  BB_CUDA(b, b->lu_err.alloc(2));
   // the solve as one CUDA graph, captured once per (precision, sweeps, tol)
   if (!b->graph || b->graph_key[0] != precision || b->graph_key[1] != sweeps || b->graph_tol != tol) {
     if (b->graph) {
       cudaGraphExecDestroy(b->graph);
       b->graph = nullptr;
     }
+    bem::BatchSolve S{};
+    const int64_t nv = b->vec.count / 3;
+    S.stream = b->stream;
+    S.sm_count = b->sm_count;
+    S.sys = b->dsys.p;
+    S.order = b->ord.p;
+    for (int i : b->order) S.N.push_back(b->hdev[i].N);
+    S.A = b->H.p;
+    S.FI = b->vec.p;
+    S.X = b->vec.p + nv;
+    S.R = b->vec.p + 2 * nv;
+    S.W = b->W.p;
+    S.dinv = b->dinv.p;
+    S.red = b->red.p;
+    S.berr = b->berr.p;
+    S.piv = b->piv.p;
+    S.perm = b->perm.p;
+    S.info = b->info.p;
+    S.conv = b->conv.p;
+    S.moved = b->moved.p;
+    S.err = b->lu_err.p;
+    S.nsys = ns;
+    const int cap = precision == BEM_PREC_FP64 ? bem::batch_lu_max_order<double>() : bem::batch_lu_max_order<float>();
+    b->lu_threads = S.N[0] <= cap ? 256 : 512;
     BB_CUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    rc = (precision == BEM_PREC_FP64) ? enqueue_solve<double>(b, precision, tol, sweeps, b->A64f.p)
-                                      : enqueue_solve<float>(b, precision, tol, sweeps, b->A32.p);
+    const bool queued = (precision == BEM_PREC_FP64) ? bem::batch_solve_enqueue<double>(S, b->A64f.p, tol, 0)
+                                                     : bem::batch_solve_enqueue<float>(S, b->A32.p, tol, sweeps);
+    rc = queued ? BEM_OK
+                : bfail(b, BEM_ERR_CUDA, std::string("batch solve launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+    b->graph_launches = S.launches;
     cudaGraph_t g = nullptr;
     cudaError_t ce = cudaStreamEndCapture(b->stream, &g);
     if (rc) {
@@ -1129,7 +590,10 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
   cudaEventElapsedTime(&ms, e0, e1);
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  b->launches += 5 + 2 * sweeps;
+  b->launches += b->graph_launches;
+  int lerr = 0;
+  BB_CUDA(b, cudaMemcpy(&lerr, b->lu_err.p, sizeof(int), cudaMemcpyDeviceToHost));
+  if (lerr != 0) return bfail(b, lerr, "batch_solve: a wait of the panel factorisation timed out");
   std::vector<int> hconv(ns), hinfo(ns);
   std::vector<double> hbe(ns);
   BB_CUDA(b, cudaMemcpy(hconv.data(), b->conv.p, ns * sizeof(int), cudaMemcpyDeviceToHost));
@@ -1147,8 +611,6 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
   }
   st.solve_seconds = ms * 1e-3;
   st.lu_threads = b->lu_threads;
-  st.lu_ms_256 = b->lu_ms[0];
-  st.lu_ms_512 = b->lu_ms[1];
   if (info) *info = st;
   b->factored = true;
   b->factored_precision = precision;

@@ -237,8 +237,8 @@ int bem_internal_points(bem_ctx* ctx, int l, const double* cx, const double* cy,
  * nrhs load cases: nrhs sets of prescribed values bc (27 x ne each, consecutive), the
  * same kode.  The systems are assembled together (one geometry launch, one persistent
  * work-queue launch for the regular pairs, one for the singular ones) and solved
- * together (one CTA per system: LU, substitution for all load cases, FP64 residual),
- * the solve captured once in a CUDA graph.  A node's prescribed displacement must be
+ * together (LU panel by panel, substitution for all load cases block by block, FP64
+ * residual, each launch over all systems), the solve captured once in a CUDA graph.  A node's prescribed displacement must be
  * the same in every element that prescribes it (BEM_ERR_MESH otherwise). */
 typedef struct bem_batch bem_batch;
 
@@ -249,8 +249,9 @@ typedef struct {
   int singular;                /* systems with an exactly zero pivot */
   double max_backward_error;   /* over the systems and their load cases */
   double solve_seconds;        /* device time of the whole solve (factor + sweeps) */
-  int lu_threads;              /* CTA size of the per-system LU picked by the autotuner */
-  float lu_ms_256, lu_ms_512;  /* the autotuner's timings of one batch LU */
+  int lu_threads;              /* CTA size of the LU: 256 panel by panel over all systems, 512
+                                  one CTA per system (a system above the cluster's capacity) */
+  float lu_ms_256, lu_ms_512;  /* no longer measured: 0 */
 } bem_batch_info;
 
 int bem_batch_create(bem_batch** batch, int device);

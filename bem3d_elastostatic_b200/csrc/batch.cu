@@ -114,7 +114,7 @@ struct bem_batch {
   std::vector<Sys> sys;
   std::vector<bem::SysDev> hdev;
   std::vector<int> order;  // systems by decreasing order
-  bool assembled = false, factored = false;
+  bool packed = false, assembled = false, factored = false;
   int factored_precision = -1;
   // device storage
   bem::DBuf<double> x, y, z, ref, tab, H, G, vec, berr, A64f;
@@ -136,7 +136,12 @@ struct bem_batch {
   double graph_tol = -1.0;
   long long graph_launches = 0;
   int lu_threads = 0;  // CTA size of the LU the solve took
+  // the solutions of the latest solve on the host (pinned), fetched with the first one asked for
+  double* host_x = nullptr;
+  size_t host_cap = 0;
+  bool host_valid = false;
   ~bem_batch() {
+    if (host_x) cudaFreeHost(host_x);
     if (graph) cudaGraphExecDestroy(graph);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -248,7 +253,7 @@ int bem_batch_add(bem_batch* b, int n, int ne, const double* x, const double* y,
   for (int i = 0; i < npins; ++i)
     if (pins[i] < 0 || pins[i] >= 3 * n) return bfail(b, BEM_ERR_ARG, "batch_add: pin out of range");
   b->sys.push_back(std::move(s));
-  b->assembled = b->factored = false;
+  b->packed = b->assembled = b->factored = b->host_valid = false;
   if (b->graph) {  // captured for the systems so far
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
@@ -256,9 +261,13 @@ int bem_batch_add(bem_batch* b, int n, int ne, const double* x, const double* y,
   return (int)b->sys.size() - 1;
 }
 
-int bem_batch_assemble(bem_batch* b) {
-  if (!b || b->sys.empty()) return bfail(b, BEM_ERR_STATE, "batch_assemble: no systems");
-  BB_CUDA(b, cudaSetDevice(b->device));
+}  // extern "C"
+
+namespace {
+
+// The systems' arrays, lists and schedules, packed and uploaded; done again only after a system
+// was added (a batch's systems do not change).
+int pack(bem_batch* b) {
   const int ns = (int)b->sys.size(), nrhs = b->nrhs;
   // host packing
   std::vector<double> hx, hy, hz;
@@ -474,6 +483,23 @@ int bem_batch_assemble(bem_batch* b) {
   }
   if ((rc = up(b, b->args, hargs)) || (rc = up(b, b->dsys, hs))) return rc;
   b->hdev = hs;
+  BB_CUDA(b, cudaStreamSynchronize(b->stream));  // the host vectors end here
+  b->packed = true;
+  return BEM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int bem_batch_assemble(bem_batch* b) {
+  if (!b || b->sys.empty()) return bfail(b, BEM_ERR_STATE, "batch_assemble: no systems");
+  BB_CUDA(b, cudaSetDevice(b->device));
+  int rc;
+  if (!b->packed && (rc = pack(b))) return rc;
+  const int ns = (int)b->sys.size();
+  const int64_t elem_off = b->total_elems;
+  const auto& hs = b->hdev;
   // geometry of every element, then H and G of every system
   if (bem::launch_geometry_arrays(b->stream, (int)elem_off, b->x.p, b->y.p, b->z.p, b->nconec.p, b->kconec_glob.p,
                                   b->ref.p, b->tab.p))
@@ -497,7 +523,7 @@ int bem_batch_assemble(bem_batch* b) {
   b->launches += 3;
   BB_CUDA(b, cudaStreamSynchronize(b->stream));
   b->assembled = true;
-  b->factored = false;
+  b->factored = b->host_valid = false;
   return BEM_OK;
 }
 
@@ -509,6 +535,7 @@ extern "C" {
 
 int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_batch_info* info) {
   if (!b || !b->assembled) return bfail(b, BEM_ERR_STATE, "batch_solve before batch_assemble");
+  b->host_valid = false;
   if (precision != BEM_PREC_FP64 && precision != BEM_PREC_FP32_IR)
     return bfail(b, BEM_ERR_ARG, "batch_solve: precision must be BEM_PREC_FP64 or BEM_PREC_FP32_IR");
   if (max_iter < 1 || max_iter > 30) return bfail(b, BEM_ERR_ARG, "batch_solve: max_iter must be in 1..30");
@@ -622,7 +649,25 @@ int bem_batch_get_solution(bem_batch* b, int i, double* x) {
     return bfail(b, BEM_ERR_ARG, "batch_get_solution: bad arguments or no solve");
   const auto& D = b->hdev[i];
   const int64_t nv = b->vec.count / 3;
-  BB_CUDA(b, cudaMemcpy(x, b->vec.p + nv + D.v_off, (size_t)D.N * D.nrhs * sizeof(double), cudaMemcpyDeviceToHost));
+  const size_t mine = (size_t)D.N * D.nrhs;
+  // one copy of all solutions instead of one per system (28 us each); large batches, or without
+  // pinned memory, directly
+  constexpr size_t kHostMost = size_t(32) << 20;  // doubles
+  if (!b->host_valid && (size_t)nv <= kHostMost) {
+    if (b->host_cap < (size_t)nv) {
+      if (b->host_x) cudaFreeHost(b->host_x);
+      b->host_x = nullptr;
+      b->host_cap = 0;
+      if (cudaMallocHost(&b->host_x, (size_t)nv * sizeof(double)) == cudaSuccess) b->host_cap = (size_t)nv;
+      else cudaGetLastError();
+    }
+    if (b->host_cap >= (size_t)nv) {
+      BB_CUDA(b, cudaMemcpy(b->host_x, b->vec.p + nv, (size_t)nv * sizeof(double), cudaMemcpyDeviceToHost));
+      b->host_valid = true;
+    }
+  }
+  if (b->host_valid) std::copy(b->host_x + D.v_off, b->host_x + D.v_off + mine, x);
+  else BB_CUDA(b, cudaMemcpy(x, b->vec.p + nv + D.v_off, mine * sizeof(double), cudaMemcpyDeviceToHost));
   return BEM_OK;
 }
 

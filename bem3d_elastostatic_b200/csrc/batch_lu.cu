@@ -5,20 +5,22 @@
 // ran on its own CTA (2,598 unknowns: 150 ms for the FP32 LU, 4 ms for one substitution of
 // eight load cases, whatever the other SMs did).  Here every launch covers one step of every
 // system that still has one, the systems ordered by size:
-//   LU, 32 columns a step (LAPACK's right-looking dgetrf):
+//   LU, two 32-column panels a step (LAPACK's right-looking dgetrf with 64 columns a step):
 //     batch_panel_kernel   the panel of a system on one cluster (panel_cluster.cuh)
-//     batch_swap_kernel    its interchanges on the other columns, and U12 = L11^{-1} A12
-//     batch_update_kernel  A22 -= L21 U12 in register-tiled FMA tiles
-//     Bound: the panel's 32 exchanges (about 35 us a step) while few systems remain, the
-//     update's traffic (the trailing matrices read and written once a step) for many.
+//     batch_swap_kernel    its interchanges on the other columns, and its rows of U12
+//     batch_update_kernel  after the first panel the second one's columns, after the second
+//                          A22 -= L21 U12, in register-tiled FMA tiles
+//     Bound: the panel's 32 exchanges (about 50 us for a system of 2,598 with four rows per
+//     thread) while few systems remain, the update's traffic (the trailing matrices read and
+//     written once a step; one panel a step moved twice as much) for many.
 //   Systems above the cluster's capacity take the one-CTA LU (batch_lu_kernel).
 //   Substitution, 128 rows a step, FP64 arithmetic on the factors, all load cases at once:
 //     the diagonal blocks are inverted once (batch_inv_kernel); at step k every block row
 //     subtracts the tile times the block solved by the step before, and block k's CTA
 //     multiplies by its inverse (batch_step_kernel).
 //   Residual: one CTA per 128 rows, the columns streamed once for all load cases.
-// Measured on 96 boxes of 78 to 2,598 unknowns with eight load cases: FP32 LU 155 -> 15.3 ms,
-// ten sweeps 42 -> 3.5 ms, residuals 15.9 -> 1.6 ms.
+// Measured on 96 boxes of 78 to 2,598 unknowns with eight load cases: FP32 LU 155 -> 16.5 ms, ten
+// sweeps 42 -> 6.8 ms, residuals 15.9 -> 2.7 ms.
 #include <algorithm>
 #include <climits>
 
@@ -69,15 +71,24 @@ __global__ void __launch_bounds__(kPanelNT, 1)
   }
 }
 
-// One column per thread: the panel's interchanges (a row of the panel's block that leaves it
-// ends where a pivot came from), then, right of the panel, the unit lower solve.
-template <typename T>
+// One column per thread: the interchanges of the panel at j0 (a row of its block that leaves it
+// ends where a pivot came from), then, from column t0 on, its rows of U12: for the second panel
+// of a step (jp = j0 - 32 the first one's columns, else -1) less the first panel's part, then
+// the unit lower solve.  part 0: all columns but the panel's own and, with jp >= 0, the first
+// panel's, which part 1 has interchanged by then.
+template <typename T, bool SECOND>
 __global__ void __launch_bounds__(128) batch_swap_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order,
-                                                         T* F, int j0, const int* __restrict__ moved) {
+                                                         T* F, int j0, int t0, int part,
+                                                         const int* __restrict__ moved) {
+  constexpr int V = 16 / sizeof(T), LP = kLuNB + V;
+  struct alignas(16) Vec {
+    T v[V];
+  };
   __shared__ int s_src[kLuNB], s_dst[kLuNB];
-  __shared__ T s_L[kLuNB][kLuNB + 1];
-  const int s = order[blockIdx.y], tid = threadIdx.x;
-  const int N = sys[s].N, w = min(kLuNB, N - j0), t0 = j0 + w;
+  __shared__ __align__(16) T s_L[kLuNB][LP];  // rows, read as 16-byte broadcasts
+  __shared__ __align__(16) T s_P[SECOND ? kLuNB : 1][LP];  // the first panel's multipliers
+  const int s = order[blockIdx.y], tid = threadIdx.x, jp = j0 - kLuNB;
+  const int N = sys[s].N, w = min(kLuNB, N - j0), b1 = j0 + w;
   if ((int)blockIdx.x * 128 >= N) return;
   const int64_t lda = sys[s].lda;
   T* A = F + sys[s].f_off;
@@ -89,42 +100,80 @@ __global__ void __launch_bounds__(128) batch_swap_kernel(const SysDev* __restric
   }
   for (int i = tid; i < kLuNB * kLuNB; i += 128) {
     const int r = i % kLuNB, c = i / kLuNB;
-    s_L[r][c] = (r < w && c < w) ? A[j0 + r + (int64_t)(j0 + c) * lda] : T(0);
+    s_L[r][c] = (r < w && c < r) ? A[j0 + r + (int64_t)(j0 + c) * lda] : T(0);
+    if (SECOND && part == 0) s_P[r][c] = r < w ? A[j0 + r + (int64_t)(jp + c) * lda] : T(0);
   }
   any = __syncthreads_or(any);
-  const int c = blockIdx.x * 128 + tid;
-  if (c >= N || (c >= j0 && c < t0) || (c < j0 && !any)) return;
+  const int c = part == 1 ? jp + tid : (int)blockIdx.x * 128 + tid;
+  if (part == 1 ? tid >= kLuNB || !any : c >= N || (c >= (SECOND ? jp : j0) && c < b1) || (c < t0 && !any)) return;
   T* col = A + (int64_t)c * lda;
+  // rows j0 .. j0 + 31: lda is a multiple of 32, so they lie in the column even where w < 32
   T x[kLuNB];
+#pragma unroll
+  for (int q = 0; q < kLuNB; q += V) {
+    const Vec v = *reinterpret_cast<const Vec*>(col + j0 + q);
+#pragma unroll
+    for (int u = 0; u < V; ++u) x[q + u] = v.v[u];
+  }
   if (any) {
-    T top[kLuNB];
+    T y[kLuNB];
 #pragma unroll
-    for (int q = 0; q < kLuNB; ++q) top[q] = q < w ? col[j0 + q] : T(0);
-#pragma unroll
-    for (int q = 0; q < kLuNB; ++q) x[q] = q < w ? col[s_src[q]] : T(0);
+    for (int q = 0; q < kLuNB; ++q) y[q] = s_src[q] < b1 ? T(0) : col[s_src[q]];
+    // rows that leave the block; within it they move between registers
 #pragma unroll
     for (int q = 0; q < kLuNB; ++q)
-      if (q < w && s_dst[q] >= t0) col[s_dst[q]] = top[q];
-  } else {
+      if (s_dst[q] >= b1) col[s_dst[q]] = x[q];
 #pragma unroll
-    for (int q = 0; q < kLuNB; ++q) x[q] = q < w ? col[j0 + q] : T(0);
+    for (int q = 0; q < kLuNB; ++q)
+      if (s_src[q] < b1 && q < w) y[q] = col[s_src[q]];  // as they were: the block is written last
+#pragma unroll
+    for (int q = 0; q < kLuNB; ++q) x[q] = q < w ? y[q] : x[q];
   }
   if (c >= t0) {
+    if constexpr (SECOND) {
+      T u1[kLuNB];
+#pragma unroll
+      for (int q = 0; q < kLuNB; q += V) {
+        const Vec v = *reinterpret_cast<const Vec*>(col + jp + q);
+#pragma unroll
+        for (int u = 0; u < V; ++u) u1[q + u] = v.v[u];
+      }
+#pragma unroll
+      for (int q = 0; q < kLuNB; ++q)
+#pragma unroll
+        for (int t = 0; t < kLuNB; t += V) {
+          const Vec l = *reinterpret_cast<const Vec*>(&s_P[q][t]);
+#pragma unroll
+          for (int u = 0; u < V; ++u) x[q] = fma(-l.v[u], u1[t + u], x[q]);
+        }
+    }
 #pragma unroll
     for (int q = 1; q < kLuNB; ++q) {
       T v = x[q];
 #pragma unroll
-      for (int t = 0; t < q; ++t) v -= s_L[q][t] * x[t];
+      for (int t = 0; t < q; t += V) {
+        const Vec l = *reinterpret_cast<const Vec*>(&s_L[q][t]);
+#pragma unroll
+        for (int u = 0; u < V; ++u)
+          if (t + u < q) v -= l.v[u] * x[t + u];
+      }
       x[q] = v;
     }
   }
 #pragma unroll
-  for (int q = 0; q < kLuNB; ++q)
-    if (q < w) col[j0 + q] = x[q];
+  for (int q = 0; q < kLuNB; q += V) {
+    Vec v;
+#pragma unroll
+    for (int u = 0; u < V; ++u) v.v[u] = x[q + u];
+    *reinterpret_cast<Vec*>(col + j0 + q) = v;
+  }
 }
 
-// Tile of 16 M x 16 M entries, M x M per thread in 16-byte vectors of rows and columns; the
-// tile of A22 is loaded with the operand tiles, so a tile costs one memory round trip.
+// A(t0.., t0..cend) -= A(t0.., j0..j0+k) A(j0..j0+k, t0..cend), k a multiple of 32: tiles of
+// 16 M x 16 M entries, M x M per thread in 16-byte vectors of rows and columns; the tile is
+// loaded with the first operand tiles, so that it costs one memory round trip.  FP32: two CTAs
+// per SM at 128 registers (one at 181 left the loads exposed: 18.9 ms for the 81 launches of the
+// batch above, 13.6 ms with two, 10.8 ms with two panels a step).
 template <typename T>
 struct UpdateTile {
   static constexpr int V = 16 / sizeof(T);           // entries per vector
@@ -132,8 +181,9 @@ struct UpdateTile {
   static constexpr int TILE = 16 * M;
 };
 template <typename T>
-__global__ void __launch_bounds__(256) batch_update_kernel(const SysDev* __restrict__ sys,
-                                                           const int* __restrict__ order, T* F, int j0) {
+__global__ void __launch_bounds__(256, 2) batch_update_kernel(const SysDev* __restrict__ sys,
+                                                           const int* __restrict__ order, T* F, int j0, int k,
+                                                              int t0, int cend) {
   using U = UpdateTile<T>;
   constexpr int V = U::V, M = U::M, TILE = U::TILE, H = M / V;
   struct alignas(16) Vec {
@@ -141,14 +191,14 @@ __global__ void __launch_bounds__(256) batch_update_kernel(const SysDev* __restr
   };
   __shared__ __align__(16) T s_a[kLuNB][TILE];
   __shared__ __align__(16) T s_b[kLuNB][TILE + V];
-  const int s = order[blockIdx.y], t0 = j0 + kLuNB;
-  const int N = sys[s].N, tiles = (N - t0 + TILE - 1) / TILE;
-  if ((int)blockIdx.x >= tiles * tiles) return;
+  const int s = order[blockIdx.y];
+  const int N = sys[s].N, tiles = (N - t0 + TILE - 1) / TILE, C = min(N, cend);
+  if ((int)blockIdx.x >= tiles * ((C - t0 + TILE - 1) / TILE)) return;
   const int64_t lda = sys[s].lda;
   T* A = F + sys[s].f_off;
   const int rb = t0 + (blockIdx.x % tiles) * TILE, cb = t0 + (blockIdx.x / tiles) * TILE;
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  // rows up to lda (a multiple of 32, zero beyond N) and columns up to N
+  // rows up to lda (a multiple of 32, zero beyond N) and columns up to C
   T acc[M][M];  // [column][row]
 #pragma unroll
   for (int j = 0; j < M; ++j) {
@@ -157,42 +207,45 @@ __global__ void __launch_bounds__(256) batch_update_kernel(const SysDev* __restr
     for (int h = 0; h < H; ++h) {
       const int r = rb + h * 16 * V + tx * V;
       Vec x{};
-      if (c < N && r < lda) x = *reinterpret_cast<const Vec*>(A + r + (int64_t)c * lda);
+      if (c < C && r < lda) x = *reinterpret_cast<const Vec*>(A + r + (int64_t)c * lda);
 #pragma unroll
       for (int u = 0; u < V; ++u) acc[j][h * V + u] = x.v[u];
     }
   }
-  for (int i = tid; i < kLuNB * TILE / V; i += 256) {
-    const int k = i / (TILE / V), r = (i % (TILE / V)) * V;
-    Vec x{};
-    if (rb + r < lda) x = *reinterpret_cast<const Vec*>(A + rb + r + (int64_t)(j0 + k) * lda);
-    *reinterpret_cast<Vec*>(&s_a[k][r]) = x;
-  }
-  for (int i = tid; i < kLuNB * TILE / V; i += 256) {
-    const int c = i / (kLuNB / V), k = (i % (kLuNB / V)) * V;
-    Vec x{};
-    if (cb + c < N) x = *reinterpret_cast<const Vec*>(A + j0 + k + (int64_t)(cb + c) * lda);
-#pragma unroll
-    for (int u = 0; u < V; ++u) s_b[k + u][c] = x.v[u];
-  }
-  __syncthreads();
-#pragma unroll 8
-  for (int k = 0; k < kLuNB; ++k) {
-    T a[M], b[M];
-#pragma unroll
-    for (int h = 0; h < H; ++h) {
-      const Vec va = *reinterpret_cast<const Vec*>(&s_a[k][h * 16 * V + tx * V]);
-      const Vec vb = *reinterpret_cast<const Vec*>(&s_b[k][h * 16 * V + ty * V]);
-#pragma unroll
-      for (int u = 0; u < V; ++u) {
-        a[h * V + u] = va.v[u];
-        b[h * V + u] = vb.v[u];
-      }
+  for (int k0 = j0; k0 < j0 + k; k0 += kLuNB) {
+    if (k0 > j0) __syncthreads();
+    for (int i = tid; i < kLuNB * TILE / V; i += 256) {
+      const int k = i / (TILE / V), r = (i % (TILE / V)) * V;
+      Vec x{};
+      if (rb + r < lda) x = *reinterpret_cast<const Vec*>(A + rb + r + (int64_t)(k0 + k) * lda);
+      *reinterpret_cast<Vec*>(&s_a[k][r]) = x;
     }
+    for (int i = tid; i < kLuNB * TILE / V; i += 256) {
+      const int c = i / (kLuNB / V), k = (i % (kLuNB / V)) * V;
+      Vec x{};
+      if (cb + c < C) x = *reinterpret_cast<const Vec*>(A + k0 + k + (int64_t)(cb + c) * lda);
 #pragma unroll
-    for (int j = 0; j < M; ++j)
+      for (int u = 0; u < V; ++u) s_b[k + u][c] = x.v[u];
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int k = 0; k < kLuNB; ++k) {
+      T a[M], b[M];
 #pragma unroll
-      for (int i = 0; i < M; ++i) acc[j][i] = fma(-a[i], b[j], acc[j][i]);
+      for (int h = 0; h < H; ++h) {
+        const Vec va = *reinterpret_cast<const Vec*>(&s_a[k][h * 16 * V + tx * V]);
+        const Vec vb = *reinterpret_cast<const Vec*>(&s_b[k][h * 16 * V + ty * V]);
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+          a[h * V + u] = va.v[u];
+          b[h * V + u] = vb.v[u];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < M; ++j)
+#pragma unroll
+        for (int i = 0; i < M; ++i) acc[j][i] = fma(-a[i], b[j], acc[j][i]);
+    }
   }
 #pragma unroll
   for (int j = 0; j < M; ++j) {
@@ -203,7 +256,7 @@ __global__ void __launch_bounds__(256) batch_update_kernel(const SysDev* __restr
       Vec x;
 #pragma unroll
       for (int u = 0; u < V; ++u) x.v[u] = acc[j][h * V + u];
-      if (c < N && r < lda) *reinterpret_cast<Vec*>(A + r + (int64_t)c * lda) = x;
+      if (c < C && r < lda) *reinterpret_cast<Vec*>(A + r + (int64_t)c * lda) = x;
     }
   }
 }
@@ -224,36 +277,55 @@ int active_from(const BatchSolve& b, int n) {
   return (int)(std::upper_bound(b.N.begin(), b.N.end(), n, [](int v, int x) { return v > x; }) - b.N.begin());
 }
 
+// the panel at j0, its interchanges and its rows of U12 from column t0 on
+template <typename T, bool SECOND>
+bool panel_and_rows(BatchSolve& b, T* F, int j0, int t0) {
+  const int maxN = b.N[0], active = active_from(b, j0 + 1), rows = maxN - j0;
+  // the fewest rows per thread (the shortest steps) with which all clusters run at once; else as
+  // many as fit, so that fewer waves of clusters are needed
+  auto ctas = [&](int l) {
+    int c = 1;
+    while (c * kPanelNT * l < rows) c *= 2;
+    return c;
+  };
+  int lpt = 1;
+  for (; lpt < kMaxLpt<T>; lpt *= 2)
+    if (ctas(lpt) <= kMaxCluster && active * ctas(lpt) <= b.sm_count) break;
+  const int C = ctas(lpt);
+  bool ok = true;
+  if (lpt == 1) ok = panel_step<T, 1>(b, F, j0, active, C);
+  else if (lpt == 2) ok = panel_step<T, 2>(b, F, j0, active, C);
+  else if constexpr (kMaxLpt<T> >= 4) ok = panel_step<T, 4>(b, F, j0, active, C);
+  if (!ok) return false;
+  if (SECOND) {  // the first panel's multipliers, which the launch below reads
+    batch_swap_kernel<T, SECOND><<<dim3(1, active), 128, 0, b.stream>>>(b.sys, b.order, F, j0, t0, 1, b.moved);
+    ++b.launches;
+  }
+  batch_swap_kernel<T, SECOND>
+      <<<dim3((maxN + 127) / 128, active), 128, 0, b.stream>>>(b.sys, b.order, F, j0, t0, 0, b.moved);
+  ++b.launches;
+  return cudaGetLastError() == cudaSuccess;
+}
+
+// A(t0.., t0..cend) -= A(t0.., j0..j0+k) A(j0..j0+k, t0..cend) of every system that reaches t0
+template <typename T>
+bool update(BatchSolve& b, T* F, int j0, int k, int t0, int cend) {
+  const int left = active_from(b, t0 + 1);
+  if (left == 0) return true;
+  constexpr int TILE = UpdateTile<T>::TILE;
+  const int rt = (b.N[0] - t0 + TILE - 1) / TILE, ct = (std::min(b.N[0], cend) - t0 + TILE - 1) / TILE;
+  batch_update_kernel<T><<<dim3(rt * ct, left), 256, 0, b.stream>>>(b.sys, b.order, F, j0, k, t0, cend);
+  ++b.launches;
+  return cudaGetLastError() == cudaSuccess;
+}
+
 template <typename T>
 bool lu_steps(BatchSolve& b, T* F) {
-  const int maxN = b.N[0];
-  for (int j0 = 0; j0 < maxN; j0 += kLuNB) {
-    const int active = active_from(b, j0 + 1), rows = maxN - j0;
-    // the fewest rows per thread (the shortest steps) with which all clusters run at once;
-    // else as many as fit, so that fewer waves of clusters are needed
-    int lpt = 1, C = 1;
-    auto ctas = [&](int l) {
-      int c = 1;
-      while (c * kPanelNT * l < rows) c *= 2;
-      return c;
-    };
-    for (lpt = 1; lpt < kMaxLpt<T>; lpt *= 2)
-      if (ctas(lpt) <= kMaxCluster && active * ctas(lpt) <= b.sm_count) break;
-    C = ctas(lpt);
-    bool ok = true;
-    if (lpt == 1) ok = panel_step<T, 1>(b, F, j0, active, C);
-    else if (lpt == 2) ok = panel_step<T, 2>(b, F, j0, active, C);
-    else if constexpr (kMaxLpt<T> >= 4) ok = panel_step<T, 4>(b, F, j0, active, C);
-    if (!ok) return false;
-    batch_swap_kernel<T><<<dim3((maxN + 127) / 128, active), 128, 0, b.stream>>>(b.sys, b.order, F, j0, b.moved);
-    ++b.launches;
-    const int left = active_from(b, j0 + kLuNB + 1);
-    if (left > 0) {
-      const int tiles = (rows - kLuNB + UpdateTile<T>::TILE - 1) / UpdateTile<T>::TILE;
-      batch_update_kernel<T><<<dim3(tiles * tiles, left), 256, 0, b.stream>>>(b.sys, b.order, F, j0);
-      ++b.launches;
-    }
-    if (cudaGetLastError() != cudaSuccess) return false;
+  for (int j0 = 0; j0 < b.N[0]; j0 += 2 * kLuNB) {
+    const int j1 = j0 + kLuNB, j2 = j1 + kLuNB;
+    if (!panel_and_rows<T, false>(b, F, j0, j1) || !update<T>(b, F, j0, kLuNB, j1, j2)) return false;
+    if (j1 >= b.N[0]) break;
+    if (!panel_and_rows<T, true>(b, F, j1, j2) || !update<T>(b, F, j0, 2 * kLuNB, j2, INT_MAX)) return false;
   }
   return true;
 }
@@ -550,20 +622,24 @@ __global__ void __launch_bounds__(256) batch_gather_kernel(const SysDev* __restr
   for (int r = 0; r < kMaxRhs; ++r) w[r] = r < S.nrhs ? R[S.v_off + p + (int64_t)r * S.N] : 0.0;
 }
 
+constexpr int kStepNT = 256;  // two threads per row
+
 // acc (8 load cases) of row tid % 128 over the half of 128 columns that tid / 128 names:
-// M(row, c) y[c], 16 loads in flight
+// M(row, c) y[c], 32 loads in flight
 template <typename T>
 __device__ __forceinline__ void tile_product(const T* M, int64_t ldm, int rows, int cols, const double (*y)[kMaxRhs],
                                              double* acc) {
   const int r = threadIdx.x % kBlk, c0 = (threadIdx.x / kBlk) * (kBlk / 2);
 #pragma unroll
   for (int q = 0; q < kMaxRhs; ++q) acc[q] = 0.0;
-  for (int c = c0; c < c0 + kBlk / 2; c += 16) {
-    T v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = (r < rows && c + u < cols) ? M[r + (int64_t)(c + u) * ldm] : T(0);
+  for (int h = 0; h < 2; ++h) {
+    const int c = c0 + 32 * h;
+    T v[32];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
+    for (int u = 0; u < 32; ++u) v[u] = (r < rows && c + u < cols) ? M[r + (int64_t)(c + u) * ldm] : T(0);
+#pragma unroll
+    for (int u = 0; u < 32; ++u) {
       const double m = (double)v[u];
 #pragma unroll
       for (int q = 0; q < kMaxRhs; ++q) acc[q] = fma(m, y[c + u][q], acc[q]);
@@ -575,10 +651,12 @@ __device__ __forceinline__ void tile_product(const T* M, int64_t ldm, int rows, 
 // tile times the block solved by the previous step, and the step's own block is solved; the
 // backward steps add their blocks to X.
 template <typename T, bool UP>
-__global__ void __launch_bounds__(256) batch_step_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order,
-                                                         const T* __restrict__ F, const double* __restrict__ dinv,
-                                                         double* __restrict__ W, double* __restrict__ X, int step,
-                                                         const int* __restrict__ conv, const int* __restrict__ info) {
+__global__ void __launch_bounds__(kStepNT, 2) batch_step_kernel(const SysDev* __restrict__ sys,
+                                                                const int* __restrict__ order, const T* __restrict__ F,
+                                                                const double* __restrict__ dinv, double* __restrict__ W,
+                                                                double* __restrict__ X, int step,
+                                                                const int* __restrict__ conv,
+                                                                const int* __restrict__ info) {
   const int s = order[blockIdx.y];
   if (conv[s] || info[s]) return;
   const SysDev& S = sys[s];
@@ -591,45 +669,47 @@ __global__ void __launch_bounds__(256) batch_step_kernel(const SysDev* __restric
   const int tid = threadIdx.x, r = tid % kBlk;
   const int rows = min(kBlk, N - i * kBlk);
   double* Wi = W + (S.piv_off + i * kBlk) * kMaxRhs;
-  double w[kMaxRhs], acc[kMaxRhs];
-#pragma unroll
-  for (int q = 0; q < kMaxRhs; ++q) w[q] = r < rows ? Wi[r * kMaxRhs + q] : 0.0;
-  // the rows' values after the subtraction, in the first half's threads
+  double acc[kMaxRhs];
+  // the rows' sums over the halves, in the first half's threads
   auto combine = [&]() {
     if (tid >= kBlk)
 #pragma unroll
       for (int q = 0; q < kMaxRhs; ++q) s_h[r][q] = acc[q];
     __syncthreads();
+    if (tid < kBlk)
 #pragma unroll
-    for (int q = 0; q < kMaxRhs; ++q) acc[q] += s_h[r][q];
+      for (int q = 0; q < kMaxRhs; ++q) acc[q] += s_h[r][q];
   };
   if (step > 0) {
     const int kp = UP ? k + 1 : k - 1, cols = min(kBlk, N - kp * kBlk);
     const double* Wk = W + (S.piv_off + kp * kBlk) * kMaxRhs;
-    for (int t = tid; t < kBlk * kMaxRhs; t += 256) (&s_y[0][0])[t] = t < cols * kMaxRhs ? Wk[t] : 0.0;
+    for (int t = tid; t < kBlk * kMaxRhs; t += kStepNT) (&s_y[0][0])[t] = t < cols * kMaxRhs ? Wk[t] : 0.0;
     __syncthreads();
     tile_product(F + S.f_off + i * kBlk + (int64_t)kp * kBlk * S.lda, S.lda, rows, cols, s_y, acc);
     combine();
+  } else {
 #pragma unroll
-    for (int q = 0; q < kMaxRhs; ++q) w[q] -= acc[q];
+    for (int q = 0; q < kMaxRhs; ++q) acc[q] = 0.0;
   }
+  if (tid < kBlk)
+#pragma unroll
+    for (int q = 0; q < kMaxRhs; ++q) acc[q] = r < rows ? Wi[r * kMaxRhs + q] - acc[q] : 0.0;
   if (i == k) {
-    __syncthreads();
+    __syncthreads();  // s_y and s_h have been read
     if (tid < kBlk)
 #pragma unroll
-      for (int q = 0; q < kMaxRhs; ++q) s_y[r][q] = w[q];
+      for (int q = 0; q < kMaxRhs; ++q) s_y[r][q] = acc[q];
     __syncthreads();
     tile_product(dinv + (2 * (S.inv_off + k) + (UP ? 1 : 0)) * (int64_t)(kBlk * kBlk), kBlk, rows, rows, s_y, acc);
-    __syncthreads();  // s_h of the subtraction has been read
     combine();
-#pragma unroll
-    for (int q = 0; q < kMaxRhs; ++q) w[q] = acc[q];
     if (UP && tid < rows)
-      for (int q = 0; q < S.nrhs; ++q) X[S.v_off + k * kBlk + r + (int64_t)q * N] += w[q];
+#pragma unroll
+      for (int q = 0; q < kMaxRhs; ++q)
+        if (q < S.nrhs) X[S.v_off + k * kBlk + r + (int64_t)q * N] += acc[q];
   }
   if (tid < rows)
 #pragma unroll
-    for (int q = 0; q < kMaxRhs; ++q) Wi[r * kMaxRhs + q] = w[q];
+    for (int q = 0; q < kMaxRhs; ++q) Wi[r * kMaxRhs + q] = acc[q];
 }
 
 template <typename T>
@@ -640,8 +720,8 @@ bool substitute(BatchSolve& b, const T* F, const double* rhs) {
   for (int up = 0; up < 2; ++up)
     for (int k = 0; k < nblk; ++k) {
       const dim3 grid(nblk - k, active_from(b, k * kBlk + 1));
-      if (up) batch_step_kernel<T, true><<<grid, 256, 0, b.stream>>>(b.sys, b.order, F, b.dinv, b.W, b.X, k, b.conv, b.info);
-      else batch_step_kernel<T, false><<<grid, 256, 0, b.stream>>>(b.sys, b.order, F, b.dinv, b.W, b.X, k, b.conv, b.info);
+      if (up) batch_step_kernel<T, true><<<grid, kStepNT, 0, b.stream>>>(b.sys, b.order, F, b.dinv, b.W, b.X, k, b.conv, b.info);
+      else batch_step_kernel<T, false><<<grid, kStepNT, 0, b.stream>>>(b.sys, b.order, F, b.dinv, b.W, b.X, k, b.conv, b.info);
       ++b.launches;
     }
   return cudaGetLastError() == cudaSuccess;

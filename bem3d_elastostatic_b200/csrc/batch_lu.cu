@@ -118,11 +118,11 @@ __global__ void __launch_bounds__(128) batch_swap_kernel(const SysDev* __restric
   if (any) {
     T y[kLuNB];
 #pragma unroll
-    for (int q = 0; q < kLuNB; ++q) y[q] = s_src[q] < b1 ? T(0) : col[s_src[q]];
+    for (int q = 0; q < kLuNB; ++q) y[q] = (q >= w || s_src[q] < b1) ? T(0) : col[s_src[q]];
     // rows that leave the block; within it they move between registers
 #pragma unroll
     for (int q = 0; q < kLuNB; ++q)
-      if (s_dst[q] >= b1) col[s_dst[q]] = x[q];
+      if (q < w && s_dst[q] >= b1) col[s_dst[q]] = x[q];
 #pragma unroll
     for (int q = 0; q < kLuNB; ++q)
       if (s_src[q] < b1 && q < w) y[q] = col[s_src[q]];  // as they were: the block is written last

@@ -1,9 +1,8 @@
 // Tensor-core GEMMs for the LU trailing update, column-major C (M x N) op= A (M x K) B (K x N).
 //
 //   dgemm_dmma_kernel   FP64 operands and accumulators on the FP64 tensor path
-//                       (mma.sync m8n8k4 .f64).  CTA tile 128x128x16, 8 warps of
-//                       64x32, cp.async double-buffered shared-memory tiles with
-//                       conflict-free pitches.
+//                       (mma.sync m8n8k4 .f64), cp.async multi-stage shared-memory
+//                       tiles with conflict-free pitches, 64 x 64 per CTA.
 //   sgemm_bf16_kernel   FP32 operands rounded to BF16 on the way into shared memory,
 //                       FP32 accumulation (mma.sync m16n8k16 .bf16, ldmatrix fragments).
 //                       SPLIT = 3 carries each operand as hi + lo BF16 parts and sums
@@ -21,17 +20,34 @@ namespace bem {
 // FP64: DMMA
 // ---------------------------------------------------------------------------------
 namespace {
-constexpr int DBM = 128, DBN = 128, DBK = 16;
-constexpr int DPA = DBM + 4;  // As[k][m] pitch (doubles)
-constexpr int DPB = DBK + 4;  // Bs[n][k] pitch (doubles)
-constexpr size_t kDmmaSmem = 2 * (DBK * DPA + DBN * DPB) * sizeof(double);
+constexpr int DBK = 16;
+
+// CTA tile BM x BN, WR x WC warps of (BM / WR) x (BN / WC), STAGES chunks of 16 k in flight.
+// As[k][m] and Bs[n][k] pitches keep the fragment loads free of bank conflicts.
+template <int BM_, int BN_, int WR_, int WC_, int STAGES_>
+struct DmmaTile {
+  static constexpr int BM = BM_, BN = BN_, WR = WR_, WC = WC_, STAGES = STAGES_;
+  static constexpr int NT = 32 * WR * WC;
+  static constexpr int PA = BM + 4, PB = DBK + 4;
+  static constexpr int TM = BM / WR / 8, TN = BN / WC / 8;  // 8 x 8 products per warp
+  static constexpr size_t SMEM = (size_t)STAGES * (DBK * PA + BN * PB) * sizeof(double);
+};
+// 64 x 64 by 4 warps at 127 registers, four CTAs per SM: with 16 warps the FP64 tensor path
+// stays busy through the other CTAs' barriers and epilogues, and small products fill the SMs.
+// Measured (TFLOP/s, K = 512, 128 x 128 tiles of 8 warps against these): 26.8 and 32.1 at
+// 11,008 x 11,008, 24.3 and 27.2 at 2,086, 12.5 and 25.6 at 1,062; K = 32, 480 x 2,598: 14.5 and
+// 10.4 us.  A third and a fourth stage gain nothing, 128 x 64 tiles lose 3 to 45 %.
+using Dmma = DmmaTile<64, 64, 2, 2, 2>;
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
@@ -40,82 +56,86 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 }
 }  // namespace
 
-template <int MODE>
-__global__ void __launch_bounds__(256, 1)
+template <int MODE, typename Tile>
+__global__ void __launch_bounds__(Tile::NT)
     dgemm_dmma_kernel(int M, int N, int K, const double* __restrict__ A, int64_t lda, const double* __restrict__ B,
                       int64_t ldb, double* C, int64_t ldc) {
+  constexpr int BM = Tile::BM, BN = Tile::BN, PA = Tile::PA, PB = Tile::PB, NT = Tile::NT, ST = Tile::STAGES;
+  constexpr int TM = Tile::TM, TN = Tile::TN;
   extern __shared__ __align__(16) double dsm[];
-  double* As = dsm;                      // [2][DBK][DPA]
-  double* Bs = dsm + 2 * DBK * DPA;      // [2][DBN][DPB]
+  double* As = dsm;                  // [ST][DBK][PA]
+  double* Bs = dsm + ST * DBK * PA;  // [ST][BN][PB]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 2) * 64;  // 2 warps along M
-  const int wn = (warp & 3) * 32;   // 4 warps along N
-  const int m0 = blockIdx.y * DBM, n0 = blockIdx.x * DBN;
+  const int wm = (warp / Tile::WC) * (BM / Tile::WR), wn = (warp % Tile::WC) * (BN / Tile::WC);
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
 
   auto load_tile = [&](int buf, int k0) {
-    double* as = As + buf * DBK * DPA;
-    double* bs = Bs + buf * DBN * DPB;
+    double* as = As + buf * DBK * PA;
+    double* bs = Bs + buf * BN * PB;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int idx = tid + 256 * i;
-      {  // A: 16 k x 64 m-pairs
-        const int k = idx >> 6, m = (idx & 63) * 2;
-        const int gm = m0 + m, gk = k0 + k;
-        int bytes = 0;
-        if (gk < K && gm < M) bytes = (gm + 1 < M) ? 16 : 8;
-        const double* src = bytes ? A + gm + (int64_t)gk * lda : A;
-        cp_async16(as + k * DPA + m, src, bytes);
-      }
-      {  // B: 128 n x 8 k-pairs
-        const int n = idx >> 3, k = (idx & 7) * 2;
-        const int gn = n0 + n, gk = k0 + k;
-        int bytes = 0;
-        if (gn < N && gk < K) bytes = (gk + 1 < K) ? 16 : 8;
-        const double* src = bytes ? B + gk + (int64_t)gn * ldb : B;
-        cp_async16(bs + n * DPB + k, src, bytes);
-      }
+    for (int i = 0; i < DBK * BM / 2 / NT; ++i) {  // A: 16 k x BM / 2 m-pairs
+      const int idx = tid + NT * i, k = idx / (BM / 2), m = (idx % (BM / 2)) * 2;
+      const int gm = m0 + m, gk = k0 + k;
+      int bytes = 0;
+      if (gk < K && gm < M) bytes = (gm + 1 < M) ? 16 : 8;
+      const double* src = bytes ? A + gm + (int64_t)gk * lda : A;
+      cp_async16(as + k * PA + m, src, bytes);
     }
-    cp_async_commit();
+#pragma unroll
+    for (int i = 0; i < BN * DBK / 2 / NT; ++i) {  // B: BN n x 8 k-pairs
+      const int idx = tid + NT * i, n = idx / (DBK / 2), k = (idx % (DBK / 2)) * 2;
+      const int gn = n0 + n, gk = k0 + k;
+      int bytes = 0;
+      if (gn < N && gk < K) bytes = (gk + 1 < K) ? 16 : 8;
+      const double* src = bytes ? B + gk + (int64_t)gn * ldb : B;
+      cp_async16(bs + n * PB + k, src, bytes);
+    }
   };
 
-  double acc[8][4][2];
+  double acc[TM][TN][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
   const int nk = (K + DBK - 1) / DBK;
-  load_tile(0, 0);
+#pragma unroll
+  for (int s = 0; s < ST - 1; ++s) {
+    if (s < nk) load_tile(s, s * DBK);
+    cp_async_commit();
+  }
+  int buf = 0;
   for (int kt = 0; kt < nk; ++kt) {
-    const int buf = kt & 1;
-    cp_async_wait_all();
-    __syncthreads();
-    if (kt + 1 < nk) load_tile(buf ^ 1, (kt + 1) * DBK);
-    const double* as = As + buf * DBK * DPA;
-    const double* bs = Bs + buf * DBN * DPB;
+    cp_async_wait<ST - 2>();
+    __syncthreads();  // chunk kt is in; every warp is past chunk kt - 1, whose buffer is refilled
+    if (kt + ST - 1 < nk) load_tile((buf + ST - 1) % ST, (kt + ST - 1) * DBK);
+    cp_async_commit();
+    const double* as = As + buf * DBK * PA;
+    const double* bs = Bs + buf * BN * PB;
 #pragma unroll
     for (int kk = 0; kk < DBK; kk += 4) {
-      double a[8], b[4];
+      double a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = as[(kk + (lane & 3)) * DPA + wm + 8 * i + (lane >> 2)];
+      for (int i = 0; i < TM; ++i) a[i] = as[(kk + (lane & 3)) * PA + wm + 8 * i + (lane >> 2)];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = bs[(wn + 8 * j + (lane >> 2)) * DPB + kk + (lane & 3)];
+      for (int j = 0; j < TN; ++j) b[j] = bs[(wn + 8 * j + (lane >> 2)) * PB + kk + (lane & 3)];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        for (int j = 0; j < TN; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
+    buf = (buf + 1) % ST;
   }
   // epilogue: two row-tiles at a time, every load of C issued before any store so the
   // read-modify-write costs one memory round trip per chunk, not one per element
 #pragma unroll
-  for (int i0 = 0; i0 < 8; i0 += 2) {
-    double old[2][4][2];
+  for (int i0 = 0; i0 < TM; i0 += 2) {
+    double old[2][TN][2];
 #pragma unroll
     for (int di = 0; di < 2; ++di) {
       const int gm = m0 + wm + 8 * (i0 + di) + (lane >> 2);
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < TN; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int gn = n0 + wn + 8 * j + 2 * (lane & 3) + h;
@@ -126,7 +146,7 @@ __global__ void __launch_bounds__(256, 1)
     for (int di = 0; di < 2; ++di) {
       const int gm = m0 + wm + 8 * (i0 + di) + (lane >> 2);
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < TN; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int gn = n0 + wn + 8 * j + 2 * (lane & 3) + h;
@@ -322,21 +342,20 @@ __global__ void __launch_bounds__(256, 1)
 // ---------------------------------------------------------------------------------
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-int gemm_dmma(bem_ctx* c, int M, int N, int K, const double* A, int64_t lda, const double* B, int64_t ldb, double* C,
-              int64_t ldc, int mode) {
-  static DeviceOnce attr;
-  if (attr.pending()) {
-    cudaFuncSetAttribute(dgemm_dmma_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem);
-    cudaFuncSetAttribute(dgemm_dmma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmmaSmem);
-    attr.mark();
-  }
-  dim3 grid((N + DBN - 1) / DBN, (M + DBM - 1) / DBM);
-  if (mode == 0)
-    dgemm_dmma_kernel<0><<<grid, 256, kDmmaSmem, c->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
-  else
-    dgemm_dmma_kernel<1><<<grid, 256, kDmmaSmem, c->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
+template <int MODE>
+static int dmma_launch(bem_ctx* c, int M, int N, int K, const double* A, int64_t lda, const double* B, int64_t ldb,
+                       double* C, int64_t ldc) {
+  static_assert(Dmma::SMEM <= 48 * 1024, "within the default dynamic shared memory");
+  const dim3 grid((N + Dmma::BN - 1) / Dmma::BN, (M + Dmma::BM - 1) / Dmma::BM);
+  dgemm_dmma_kernel<MODE, Dmma><<<grid, Dmma::NT, Dmma::SMEM, c->stream>>>(M, N, K, A, lda, B, ldb, C, ldc);
   BEM_LAUNCH_CHECK(c);
   return BEM_OK;
+}
+
+int gemm_dmma(bem_ctx* c, int M, int N, int K, const double* A, int64_t lda, const double* B, int64_t ldb, double* C,
+              int64_t ldc, int mode) {
+  return mode == 0 ? dmma_launch<0>(c, M, N, K, A, lda, B, ldb, C, ldc)
+                   : dmma_launch<1>(c, M, N, K, A, lda, B, ldb, C, ldc);
 }
 
 int gemm_bf16(bem_ctx* c, int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb, float* C,

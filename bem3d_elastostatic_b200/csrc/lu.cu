@@ -1226,6 +1226,10 @@ namespace {
 
 // FP64 sub-panels with as many lines as one cluster holds go to panel64.cu; wider ones and
 // the FP32 ones to the grid-synchronised panel_kernel.
+bool on_cluster(const LUWorkspace& ws, int lines) {
+  return 2 * ws.gmax >= 2 * kPanelW && lines <= panel_cluster_lines();
+}
+
 // The barrier counter grows monotonically over a factorisation (zeroed once with the
 // status words); each launch waits for its own arrivals on top of bar_base.
 template <typename T>
@@ -1234,7 +1238,7 @@ int panel_launch(bem_ctx* c, const LUWorkspace& ws, T* S, int64_t lda, int n, in
   static DeviceOnce checked;  // per instantiation (T) and device
   const int cols = n - r0;
   if constexpr (sizeof(T) == 8)
-    if (cols <= panel_cluster_lines()) return panel_cluster_launch(c, S, lda, n, r0, w, piv, ws.status);
+    if (on_cluster(ws, cols)) return panel_cluster_launch(c, S, lda, n, r0, w, piv, ws.status, ws.cand_idx);
   static const int cap = [] {  // BEM_PANEL_CTAS: at most this many CTAs per panel launch
     const char* e = getenv("BEM_PANEL_CTAS");
     return e ? std::max(1, atoi(e)) : INT_MAX;
@@ -1498,6 +1502,20 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
         return rc;
       }
       prof.end(c->stream);
+      if constexpr (sizeof(T) == 8)
+        if (!window && on_cluster(ws, n - r0)) {
+          // its interchanges and the solve of the panel's rows below in one launch
+          const int q0 = r0 + w, q1 = j0 + jb;
+          prof.begin(1, c->stream);
+          if ((rc = panel_rows_launch(c, S, lda, n, r0, w, q1, ws.cand_idx))) return rc;
+          prof.end(c->stream);
+          prof.begin(2, c->stream);
+          if (q1 > q0 && (rc = gemm<T>(c, q1 - q0, n - q0, w, S + q0 + (int64_t)r0 * lda, lda,
+                                       S + r0 + (int64_t)q0 * lda, lda, S + q0 + (int64_t)q0 * lda, lda, 0)))
+            return rc;
+          prof.end(c->stream);
+          continue;
+        }
       prof.begin(1, c->stream);
       // swaps on every other row of S: the earlier panels' multipliers (rows [0, r0),
       // so that the factors end up as T = P L U) and the trailing rows; with window

@@ -27,7 +27,7 @@ constexpr int kPanelW = 32;  // columns of T factored by one cooperative panel l
 // allocates it per call; lu_factor_ws() takes it from the caller.
 struct LUWorkspace {
   double* cand_val;   // [2][gmax]
-  int* cand_idx;      // [2][gmax]
+  int* cand_idx;      // [2][gmax] (the cluster panel: its interchanges, 64 ints)
   void* cand_col;     // [2][gmax][kPanelW] of T
   void* diag_col;     // [2][kPanelW] of T
   unsigned* barrier;  // grid-barrier counter (zeroed before every panel launch)
@@ -59,7 +59,8 @@ int lu_solve_ws(bem_ctx* c, const T* S, int64_t lda, int n, const int* perm, dou
 
 // the FP64 sub-panel on one cluster (panel64.cu)
 int panel_cluster_lines();
-int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status);
+int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status, int* moved);
+int panel_rows_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int q1, const int* moved);
 
 template <typename T>
 int lu_factor(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int nb, int* info);

@@ -17,6 +17,7 @@ struct PanelArgs {
   double* S;
   int64_t lda;
   int* status;  // [0] error code, [1] info
+  int* moved;   // [q]: the line that ends at position r0 + q; [32 + q]: where line r0 + q ends
 };
 
 template <int LPT, int NT>
@@ -43,8 +44,69 @@ __global__ void __launch_bounds__(NT, 1) panel_cluster_kernel(PanelArgs P, int C
     if (tid == 0) atomicCAS(P.status, 0, BEM_ERR_TIMEOUT);
     return;
   }
+  for (int c = tid; c < nl; c += NT) {
+    const int p = sm.pos[c], line = base + c;
+    if (p < r0 + w) P.moved[p - r0] = line;
+    if (line < r0 + w) P.moved[kPanelW + line - r0] = p;
+  }
   for (int c = wp; c < nl; c += NW)
     if (lane < w) P.S[(int64_t)sm.pos[c] * P.lda + r0 + lane] = sm.val[lane * Sm::kPitchL + c];
+}
+
+// One row of S per thread, outside the sub-panel: its interchanges (a column of the sub-panel
+// that leaves it ends where a pivot came from), all loads before the first store, and for the
+// panel's rows below, [r0 + w, q1), the solve with the unit upper triangle of S(r0.., r0..).
+// (The interchanges one after the other, each a dependent exchange, and a launch of its own for
+// the solve took 9.5 us where this takes 6.)
+__global__ void __launch_bounds__(128) panel_rows_kernel(double* S, int64_t lda, int n, int r0, int w, int q1,
+                                                         const int* __restrict__ moved) {
+  constexpr int W = kPanelW;
+  __shared__ int s_src[W], s_dst[W];
+  __shared__ __align__(16) double s_U[W][W + 2];  // [column][row], read as 16-byte broadcasts
+  const int tid = threadIdx.x, b1 = r0 + w;
+  bool any = false;
+  if (tid < W) {
+    s_src[tid] = tid < w ? moved[tid] : r0 + tid;
+    s_dst[tid] = tid < w ? moved[W + tid] : r0 + tid;
+    any = s_src[tid] != r0 + tid;
+  }
+  for (int i = tid; i < W * W; i += 128) {
+    const int a = i % W, b = i / W;
+    s_U[b][a] = (b < w && a < b) ? S[r0 + a + (int64_t)(r0 + b) * lda] : 0.0;
+  }
+  any = __syncthreads_or(any);
+  const int i = blockIdx.x * 128 + tid, r = i < r0 ? i : i + w;
+  const bool solve = r >= b1 && r < q1;
+  if (r >= n || (!any && !solve)) return;
+  double x[W];
+#pragma unroll
+  for (int q = 0; q < W; ++q) x[q] = q < w ? S[r + (int64_t)(r0 + q) * lda] : 0.0;
+  if (any) {
+    double y[W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) y[q] = q < w ? S[r + (int64_t)s_src[q] * lda] : 0.0;
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+      if (q < w && s_dst[q] >= b1) S[r + (int64_t)s_dst[q] * lda] = x[q];
+#pragma unroll
+    for (int q = 0; q < W; ++q) x[q] = y[q];
+  }
+  if (solve) {
+#pragma unroll
+    for (int b = 1; b < W; ++b) {
+      double v = x[b];
+#pragma unroll
+      for (int a = 0; a < b; a += 2) {
+        const double2 u = *reinterpret_cast<const double2*>(&s_U[b][a]);
+        v = fma(-x[a], u.x, v);
+        if (a + 1 < b) v = fma(-x[a + 1], u.y, v);
+      }
+      x[b] = v;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < W; ++q)
+    if (q < w) S[r + (int64_t)(r0 + q) * lda] = x[q];
 }
 
 template <int LPT, int NT>
@@ -73,15 +135,24 @@ int panel_cluster_lines() {
 }
 
 // The sub-panel rows [r0, r0 + w) of S, pivoting over the columns [r0, n): n - r0 at most
-// panel_cluster_lines().
-int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status) {
-  const PanelArgs P{{n, r0, w, piv, status + 1, c->wait_ns}, S, lda, status};
+// panel_cluster_lines().  moved (64 ints) receives its interchanges as panel_rows takes them.
+int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status,
+                         int* moved) {
+  const PanelArgs P{{n, r0, w, piv, status + 1, c->wait_ns}, S, lda, status, moved};
   const int lines = n - r0;
   if (lines > kMaxCluster * 512) return launch<2, 384>(c, P, kMaxCluster);
   if (lines > kMaxCluster * 256) return launch<1, 512>(c, P, kMaxCluster);
   int C = 1;
   while (C * 256 < lines) C *= 2;
   return launch<1, 256>(c, P, C);
+}
+
+// The sub-panel's interchanges on every other row of S and the solve of the rows [r0 + w, q1).
+int panel_rows_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int q1, const int* moved) {
+  if (n == w) return BEM_OK;
+  panel_rows_kernel<<<(n - w + 127) / 128, 128, 0, c->stream>>>(S, lda, n, r0, w, q1, moved);
+  BEM_LAUNCH_CHECK(c);
+  return BEM_OK;
 }
 
 }  // namespace bem

@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(kTriThreads) batch_inv_kernel(const SysDev* __
                                                                 const T* __restrict__ F, double* __restrict__ dinv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* U = reinterpret_cast<double*>(smem_raw);
+  constexpr int P = kTriPitch<double>;
   __shared__ double dg[kBlk];
   const SysDev& S = sys[blockIdx.z];
   const int k0 = blockIdx.x * kBlk, m = min(kBlk, S.N - k0);
@@ -591,18 +592,18 @@ __global__ void __launch_bounds__(kTriThreads) batch_inv_kernel(const SysDev* __
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       const int i = (base + u * kTriThreads) % kBlk, j = (base + u * kTriThreads) / kBlk;
-      if (lower) U[j + i * kTriPitch] = v[u];
-      else U[i + j * kTriPitch] = i < j ? v[u] / dg[i] : 0.0;
+      if (lower) U[j + i * P] = v[u];
+      else U[i + j * P] = i < j ? v[u] / dg[i] : 0.0;
     }
   }
-  unit_upper_inverse(U, U + 128 * kTriPitch);
+  unit_upper_inverse<double, kTriThreads>(U, U + 128 * P);
   double* V = dinv + (2 * (S.inv_off + blockIdx.x) + blockIdx.y) * (int64_t)(kBlk * kBlk);
   for (int idx = tid; idx < kBlk * kBlk; idx += kTriThreads) {
     const int i = idx % kBlk, j = idx / kBlk;
     double v = 0.0;
     if (i < m && j < m) {
-      if (lower) v = j <= i ? U[j + i * kTriPitch] : 0.0;
-      else v = i <= j ? U[i + j * kTriPitch] / dg[j] : 0.0;
+      if (lower) v = j <= i ? U[j + i * P] : 0.0;
+      else v = i <= j ? U[i + j * P] / dg[j] : 0.0;
     }
     V[idx] = v;
   }
@@ -864,7 +865,7 @@ __global__ void batch_copy_kernel(const SysDev* __restrict__ sys, const double* 
 template <typename T>
 bool attributes(size_t perm_smem) {
   return cudaFuncSetAttribute(batch_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(kTriDoubles * sizeof(double))) == cudaSuccess &&
+                              (int)(kTriElems<double> * sizeof(double))) == cudaSuccess &&
          cudaFuncSetAttribute(batch_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem) ==
              cudaSuccess;
 }
@@ -908,7 +909,7 @@ bool batch_solve_enqueue(BatchSolve& b, T* F, double tol, int sweeps) {
     ++b.launches;
   }
   batch_perm_kernel<<<b.nsys, 256, perm_smem, b.stream>>>(b.sys, b.piv, b.perm);
-  batch_inv_kernel<T><<<dim3(nblk, 2, b.nsys), kTriThreads, kTriDoubles * sizeof(double), b.stream>>>(b.sys, F, b.dinv);
+  batch_inv_kernel<T><<<dim3(nblk, 2, b.nsys), kTriThreads, kTriElems<double> * sizeof(double), b.stream>>>(b.sys, F, b.dinv);
   batch_start_kernel<<<dim3((maxN + 255) / 256, b.nsys), 256, 0, b.stream>>>(b.sys, b.FI, b.X, b.R, b.berr);
   b.launches += 3;
   if (cudaGetLastError() != cudaSuccess) return false;

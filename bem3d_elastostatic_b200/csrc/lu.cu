@@ -22,6 +22,7 @@
 #include <atomic>
 #include <vector>
 
+#include "grid_sync.cuh"
 #include "lu.cuh"
 #include "tri_inv.cuh"
 
@@ -32,26 +33,6 @@ constexpr int kInvBlock = 128;       // unit-triangle inverse block of the block
 constexpr int kSolveBlock = 128;     // diagonal block of the triangular solves
 constexpr int kPanelSmemMax = 200 * 1024;  // dynamic shared memory of a panel CTA
 constexpr int kSweepThreads = 512;   // threads of a triangular sweep CTA (4 per row of a block)
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
 
 __device__ __forceinline__ void better(double& bv, int& bc, int& bg, double v, int cidx, int gidx) {
   if (v > bv || (v == bv && cidx < bc)) {
@@ -559,34 +540,6 @@ __global__ void __launch_bounds__(kBlockThreads) window_block_kernel(float* S, i
   }
 }
 
-// Grid barrier of a cooperative launch (bounded): every thread's earlier writes are
-// ordered before the arrival (CTA barrier, then thread 0's fence and release); the
-// wait gives up after wait_ns or once another CTA recorded an error, and records
-// BEM_ERR_TIMEOUT.  Returns false when the launch must stop.
-__device__ __forceinline__ bool coop_barrier(unsigned* barrier, unsigned target, int* status,
-                                             unsigned long long wait_ns, int* s_abort) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    red_release_add_u32(barrier, 1u);
-    const unsigned long long t0 = globaltimer_ns();
-    unsigned spins = 0;
-    int abort = 0;
-    while (ld_acquire_u32(barrier) < target) {
-      if ((++spins & 63u) == 0 && (globaltimer_ns() - t0 > wait_ns || *((volatile int*)status) != 0)) {
-        abort = 1;
-        break;
-      }
-      __nanosleep(32);
-    }
-    if (abort) atomicCAS(status, 0, BEM_ERR_TIMEOUT);
-    __threadfence();
-    *s_abort = abort;
-  }
-  __syncthreads();
-  return *s_abort == 0;
-}
-
 // The diagonal block [j0, t0)^2 of a window-pivoted FP32 panel in one cooperative
 // launch: the 32-wide sub-panels in turn, each in three phases separated by grid
 // barriers (two per sub-panel) instead of kernel boundaries:
@@ -891,166 +844,18 @@ __global__ void trsm_small_kernel(T* S, int64_t lda, int k0, int w, int r_lo, in
 
 // V[b] = inverse of the unit upper triangle of diagonal block b of S11 (jb x jb, blocks of
 // 128), column-major with leading dimension 128; one CTA per block.
-__global__ void __launch_bounds__(kTriThreads) inv_unit_upper_f64_kernel(const double* S11, int64_t lda, int jb,
-                                                                         double* V) {
+template <typename T>
+__global__ void __launch_bounds__(kTriThreads) inv_unit_upper_kernel(const T* S11, int64_t lda, int jb, T* V) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* U = reinterpret_cast<double*>(smem_raw);
+  constexpr int P = kTriPitch<T>;
+  T* U = reinterpret_cast<T*>(smem_raw);
   const int o = kInvBlock * blockIdx.x, m = min(kInvBlock, jb - o);
-  stage_block<double>(U, kTriPitch, S11 + o + (int64_t)o * lda, lda, m, m, kInvBlock, kInvBlock,
-                      [](int a, int b) { return a < b; });
-  unit_upper_inverse(U, U + 128 * kTriPitch);
-  double* Vb = V + (size_t)blockIdx.x * kInvBlock * kInvBlock;
+  stage_block<T>(U, P, S11 + o + (int64_t)o * lda, lda, m, m, kInvBlock, kInvBlock,
+                 [](int a, int b) { return a < b; });
+  unit_upper_inverse<T, kTriThreads>(U, U + 128 * P);
+  T* Vb = V + (size_t)blockIdx.x * kInvBlock * kInvBlock;
   for (int idx = threadIdx.x; idx < kInvBlock * kInvBlock; idx += kTriThreads)
-    Vb[idx] = U[idx % kInvBlock + (idx / kInvBlock) * kTriPitch];
-}
-
-// The inverse of a unit upper triangle for FP32 factors with U and V both in shared memory
-// (2 x 64 KB), blocked by 32: four warps invert the diagonal blocks (lane j holds column j of
-// its block in registers and back-substitutes), then the off-diagonal blocks follow in order
-// of their distance from the diagonal, V_ij = -V_ii * sum_{k=i+1..j} U_ik V_kj, the
-// off-diagonal blocks of one distance from the diagonal computed together (two
-// barriers per distance); V is written to global memory once at the end.
-constexpr int kInvThreads = 512;
-
-// V (zeroed, [128][128] column-major, shared) := U^{-1} for the unit upper triangle whose
-// strict upper part U holds (shared, zero elsewhere), jb <= 128; all threads take part.
-__device__ __forceinline__ void unit_upper_inverse_smem(const float* U, float* V, int jb, float (*tmp)[32 * 33]) {
-  constexpr int B = 32, NB = 128;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nblk = (jb + B - 1) / B;
-  if (warp < nblk) {
-    const int o = warp * B;
-    float x[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-    for (int i = B - 2; i >= 0; --i) {
-      float sacc = x[i];
-#pragma unroll
-      for (int k = i + 1; k < B; ++k) sacc -= U[(o + i) + (o + k) * NB] * x[k];
-      x[i] = (i < lane) ? sacc : x[i];
-    }
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-      if (o + i < jb && o + lane < jb) V[(o + i) + (o + lane) * NB] = x[i];
-  }
-  __syncthreads();
-  for (int d = 1; d < nblk; ++d) {
-    const int nb_d = nblk - d;  // blocks (bi, bi + d)
-    for (int e = tid; e < nb_d * B * B; e += kInvThreads) {
-      const int bi = e / (B * B), r = e % B, cc = (e / B) % B;
-      const int oi = bi * B, oj = (bi + d) * B;
-      float acc = 0.f;
-      for (int k = oi + B; k <= oj + B - 1 && k < jb; ++k) acc += U[(oi + r) + k * NB] * V[k + (oj + cc) * NB];
-      tmp[bi][r + cc * 33] = acc;
-    }
-    __syncthreads();
-    for (int e = tid; e < nb_d * B * B; e += kInvThreads) {
-      const int bi = e / (B * B), r = e % B, cc = (e / B) % B;
-      const int oi = bi * B, oj = (bi + d) * B;
-      float acc = 0.f;
-#pragma unroll 8
-      for (int k = 0; k < B; ++k) acc += V[(oi + r) + (oi + k) * NB] * tmp[bi][k + cc * 33];
-      if (oi + r < jb && oj + cc < jb) V[(oi + r) + (oj + cc) * NB] = -acc;
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kInvThreads) inv_unit_upper_f32_kernel(const float* S11, int64_t lda, int jb,
-                                                                         float* Vout, int ldv) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int B = 32, NB = 128, NBLK = NB / B;
-  float* U = reinterpret_cast<float*>(smem_raw);  // [NB][NB] column-major, the strict upper part
-  float* V = U + NB * NB;                         // [NB][NB] column-major
-  __shared__ float tmp[NBLK - 1][B * 33];
-  stage_block<float>(U, NB, S11, lda, jb, jb, NB, NB, [](int a, int b) { return a < b; });
-  for (int i = threadIdx.x; i < NB * NB; i += kInvThreads) V[i] = 0.f;
-  __syncthreads();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nblk = (jb + B - 1) / B;
-  if (warp < nblk) {
-    const int o = warp * B;
-    float x[B];
-#pragma unroll
-    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? 1.f : 0.f;
-#pragma unroll
-    for (int i = B - 2; i >= 0; --i) {
-      float sacc = x[i];
-#pragma unroll
-      for (int k = i + 1; k < B; ++k) sacc -= U[(o + i) + (o + k) * NB] * x[k];
-      x[i] = (i < lane) ? sacc : x[i];
-    }
-#pragma unroll
-    for (int i = 0; i < B; ++i)
-      if (o + i < jb && o + lane < jb) V[(o + i) + (o + lane) * NB] = x[i];
-  }
-  __syncthreads();
-  for (int d = 1; d < nblk; ++d) {
-    const int nb_d = nblk - d;  // blocks (bi, bi + d)
-    for (int e = tid; e < nb_d * B * B; e += kInvThreads) {
-      const int bi = e / (B * B), r = e % B, cc = (e / B) % B;
-      const int oi = bi * B, oj = (bi + d) * B;
-      float acc = 0.f;
-      for (int k = oi + B; k <= oj + B - 1 && k < jb; ++k) acc += U[(oi + r) + k * NB] * V[k + (oj + cc) * NB];
-      tmp[bi][r + cc * 33] = acc;
-    }
-    __syncthreads();
-    for (int e = tid; e < nb_d * B * B; e += kInvThreads) {
-      const int bi = e / (B * B), r = e % B, cc = (e / B) % B;
-      const int oi = bi * B, oj = (bi + d) * B;
-      float acc = 0.f;
-#pragma unroll 8
-      for (int k = 0; k < B; ++k) acc += V[(oi + r) + (oi + k) * NB] * tmp[bi][k + cc * 33];
-      if (oi + r < jb && oj + cc < jb) V[(oi + r) + (oj + cc) * NB] = -acc;
-    }
-    __syncthreads();
-  }
-  for (int i = tid; i < jb * jb; i += kInvThreads) {
-    const int r = i % jb, cc = i / jb;
-    Vout[r + (int64_t)cc * ldv] = V[r + cc * NB];
-  }
-}
-
-// The inverses a window-pivoted panel's TRSMs take, for every 128-block b of the
-// panel's diagonal block (S11 = S(j0.., j0..), jb <= 512): blockIdx.y = 0 writes
-// Vu[b] = the inverse of the unit upper triangle of block b (the multipliers, as
-// inv_unit_upper_f32_kernel), blockIdx.y = 1 writes Wl[b] = the inverse of its lower
-// triangle, diagonal included (U^T of T).  The lower inverse goes through the unit
-// upper routine: W = Lu D with Lu unit lower, so W^{-1} = D^{-1} ((Lu^T)^{-1})^T.
-// Each inverse is 128 x 128 column-major (leading dimension 128, zero outside jb x jb).
-__global__ void __launch_bounds__(kInvThreads) panel_inv_f32_kernel(const float* S11, int64_t lda, int jb,
-                                                                    float* Vu, float* Wl) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int B = 32, NB = 128, NBLK = NB / B;
-  float* U = reinterpret_cast<float*>(smem_raw);
-  float* V = U + NB * NB;
-  __shared__ float tmp[NBLK - 1][B * 33];
-  __shared__ float rdiag[NB];
-  const int b = blockIdx.x, o = b * NB, bb = min(NB, jb - o);
-  const float* D = S11 + o + (int64_t)o * lda;
-  const bool lower = blockIdx.y == 1;
-  if (!lower) {
-    stage_block<float>(U, NB, D, lda, bb, bb, NB, NB, [](int a, int c) { return a < c; });
-  } else {
-    for (int i = threadIdx.x; i < NB; i += kInvThreads) rdiag[i] = (i < bb) ? D[i + (int64_t)i * lda] : 1.f;
-    __syncthreads();
-    // U[a][c] = Lu^T[a][c] = W[c][a] / W[a][a]  (a < c)
-    for (int i = threadIdx.x; i < NB * NB; i += kInvThreads) {
-      const int a = i % NB, c = i / NB;
-      U[i] = (a < c && c < bb) ? D[c + (int64_t)a * lda] / rdiag[a] : 0.f;
-    }
-  }
-  for (int i = threadIdx.x; i < NB * NB; i += kInvThreads) V[i] = 0.f;
-  __syncthreads();
-  unit_upper_inverse_smem(U, V, bb, tmp);
-  float* out = (lower ? Wl : Vu) + (size_t)b * NB * NB;
-  for (int i = threadIdx.x; i < NB * NB; i += kInvThreads) {
-    const int r = i % NB, c = i / NB;
-    float v = 0.f;
-    if (r < bb && c < bb) v = lower ? ((r >= c) ? V[c + r * NB] / rdiag[r] : 0.f) : V[r + c * NB];
-    out[i] = v;
-  }
+    Vb[idx] = U[idx % kInvBlock + (idx / kInvBlock) * P];
 }
 
 // ---------------------------------------------------------------------------------
@@ -1357,21 +1162,18 @@ struct LUProfile {
 
 static size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
-// blocks of the TRSM-inverse region: FP32 factors keep both triangles' inverses of every
-// diagonal block of a panel (panel_inv_f32_kernel), FP64 the upper ones
-static size_t inv_blocks(int elem, int nb) {
-  return (elem == 4 ? 2 : 1) * (size_t)((nb + kInvBlock - 1) / kInvBlock);
-}
+// blocks of the TRSM-inverse region: the unit upper inverses of a panel's diagonal blocks
+static size_t inv_blocks(int nb) { return (size_t)((nb + kInvBlock - 1) / kInvBlock); }
 
 static size_t finv_count(int elem, int nb) {
-  return elem == 4 ? 2 * (size_t)nb * nb + 2 * (size_t)nb * kInvBlock : 0;
+  return elem == 4 ? 2 * (size_t)nb * nb : 0;
 }
 
 size_t lu_workspace_bytes(int n, int nb, int gmax, int elem) {
   const size_t ldy = ((size_t)n + 31) / 32 * 32;
   return up256(2 * (size_t)gmax * sizeof(double)) + up256(2 * (size_t)gmax * sizeof(int)) +
          up256(2 * (size_t)gmax * kPanelW * elem) + up256(2 * (size_t)kPanelW * elem) + up256(16) +
-         up256(inv_blocks(elem, nb) * kInvBlock * kInvBlock * elem) + up256(finv_count(elem, nb) * elem) +
+         up256(inv_blocks(nb) * kInvBlock * kInvBlock * elem) + up256(finv_count(elem, nb) * elem) +
          up256(ldy * nb * elem);
 }
 
@@ -1392,7 +1194,7 @@ LUWorkspace lu_workspace_carve(void* base, int n, int nb, int gmax, int elem) {
   w.status = reinterpret_cast<int*>(p + 8);
   p += up256(16);
   w.inv = p;
-  p += up256(inv_blocks(elem, nb) * kInvBlock * kInvBlock * elem);
+  p += up256(inv_blocks(nb) * kInvBlock * kInvBlock * elem);
   w.finv = finv_count(elem, nb) ? p : nullptr;
   p += up256(finv_count(elem, nb) * elem);
   w.ybuf = p;
@@ -1440,12 +1242,8 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
   // window pivoting (pivot search within each sub-panel's diagonal block) or partial
   // pivoting (over every remaining row of T)
   const bool window = c->lu_window;
-  const size_t inv_smem = kTriDoubles * sizeof(double);
-  cudaFuncSetAttribute(inv_unit_upper_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
-  cudaFuncSetAttribute(inv_unit_upper_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(2 * kInvBlock * kInvBlock * sizeof(float)));
-  cudaFuncSetAttribute(panel_inv_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(2 * kInvBlock * kInvBlock * sizeof(float)));
+  const size_t inv_smem = kTriElems<T> * sizeof(T);
+  cudaFuncSetAttribute(inv_unit_upper_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
   int rc;
   // window-pivoted FP32 panels: the diagonal block in one cooperative launch
   // (panel_coop_kernel; BEM_PANEL_COOP=0 selects a launch pair per sub-panel)
@@ -1555,67 +1353,17 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
     }
     if (t0 < n) {
       const int m = n - t0;
-      const int nib = (nb + kInvBlock - 1) / kInvBlock;
-      T* Vu = V;                                          // [nib][128 x 128]
-      T* Wl = V + (size_t)(kInvBlock * kInvBlock) * nib;  // [nib][128 x 128]
-      // blocked panels (FP32): jb x jb inverses of the unit upper and the lower triangle,
-      // and a jb x 128 scratch for each
+      // blocked panels (FP32): jb x jb inverses of the unit upper and the lower triangle
       T* XU = blocked ? reinterpret_cast<T*>(ws.finv) : nullptr;
       T* XL = blocked ? XU + (size_t)jb * jb : nullptr;
-      T* Tu = blocked ? XL + (size_t)jb * jb : nullptr;
-      T* Tl = blocked ? Tu + (size_t)jb * kInvBlock : nullptr;
       if (blocked) {
-        // the panel's diagonal-block inverses: the 128 x 128 ones, then the two full
-        // triangles' block column by block column (U unit upper, W lower, both of the
-        // panel's diagonal block of S):
-        //   XU_{<b,b} = -(XU_{<b,<b} U_{<b,b}) inv(U_bb),  XL_{b,<b} = -inv(W_bb) (W_{b,<b} XL_{<b,<b});
-        // then the rest of the sub-panels' columns in one product, B = S(j0..t0, t0..n)
-        // := W^{-1} B, through the TRSM buffer
+        // both triangles' inverses of the panel's diagonal block, then the rest of the
+        // sub-panels' columns in one product, B = S(j0..t0, t0..n) := W^{-1} B
         prof.begin(2, c->stream);
-        const int nblk = (jb + kInvBlock - 1) / kInvBlock;
-        panel_inv_f32_kernel<<<dim3(nblk, 2), kInvThreads, 2 * kInvBlock * kInvBlock * sizeof(float), c->stream>>>(
-            reinterpret_cast<const float*>(S + j0 + (int64_t)j0 * lda), lda, jb, reinterpret_cast<float*>(Vu),
-            reinterpret_cast<float*>(Wl));
-        BEM_LAUNCH_CHECK(c);
-        BEM_CUDA(c, cudaMemsetAsync(XU, 0, 2 * (size_t)jb * jb * sizeof(T), c->stream));
-        // the two inverses are independent: XU's chain (no tcgen05 GEMM, whose operand
-        // buffer is the context's) runs on the auxiliary stream, joined before the
-        // block-row TRSM that needs it; XL's chain and the L21 product run here
-        cudaStream_t main_stream = c->stream;
-        const bool fork = c->aux_stream != nullptr;
-        if (fork) {
-          BEM_CUDA(c, cudaEventRecord(c->ev_fork, main_stream));
-          BEM_CUDA(c, cudaStreamWaitEvent(c->aux_stream, c->ev_fork, 0));
-          c->stream = c->aux_stream;
-        }
-        rc = 0;
-        for (int b0 = 0; b0 < jb && rc == 0; b0 += kInvBlock) {
-          const int bb = std::min(kInvBlock, jb - b0);
-          const T* Vb = Vu + (size_t)(b0 / kInvBlock) * kInvBlock * kInvBlock;
-          if (cudaMemcpy2DAsync(XU + b0 + (size_t)b0 * jb, jb * sizeof(T), Vb, kInvBlock * sizeof(T), bb * sizeof(T),
-                                bb, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess) {
-            rc = bem_fail(c, BEM_ERR_CUDA, "inverse assembly copy failed");
-          } else if (b0 > 0) {
-            rc = gemm<T>(c, b0, bb, b0, XU, jb, S + j0 + (int64_t)(j0 + b0) * lda, lda, Tu, jb, 1);
-            if (rc == 0) rc = gemm<T>(c, b0, bb, bb, Tu, jb, Vb, kInvBlock, XU + (size_t)b0 * jb, jb, 0);
-          }
-        }
-        if (fork) {
-          if (rc == 0 && cudaEventRecord(c->ev_join, c->aux_stream) != cudaSuccess)
-            rc = bem_fail(c, BEM_ERR_CUDA, "event record failed");
-          c->stream = main_stream;
-        }
-        if (rc) return rc;
-        for (int b0 = 0; b0 < jb; b0 += kInvBlock) {
-          const int bb = std::min(kInvBlock, jb - b0);
-          const T* Wb = Wl + (size_t)(b0 / kInvBlock) * kInvBlock * kInvBlock;
-          BEM_CUDA(c, cudaMemcpy2DAsync(XL + b0 + (size_t)b0 * jb, jb * sizeof(T), Wb, kInvBlock * sizeof(T),
-                                        bb * sizeof(T), bb, cudaMemcpyDeviceToDevice, c->stream));
-          if (b0 == 0) continue;
-          if ((rc = gemm<T>(c, bb, b0, b0, S + (j0 + b0) + (int64_t)j0 * lda, lda, XL, jb, Tl, kInvBlock, 1)) ||
-              (rc = gemm<T>(c, bb, b0, bb, Wb, kInvBlock, Tl, kInvBlock, XL + b0, jb, 0)))
-            return rc;
-        }
+        if ((rc = panel_inverses_launch(c, reinterpret_cast<const float*>(S + j0 + (int64_t)j0 * lda), lda, jb,
+                                        reinterpret_cast<float*>(XU), reinterpret_cast<float*>(XL), ws.barrier,
+                                        bar_base, ws.status)))
+          return rc;
         float* L21 = reinterpret_cast<float*>(S + j0 + (int64_t)t0 * lda);
         if (gemm_tri_in_place(c, jb, m, jb, L21, lda)) {  // written over its own operand
           if ((rc = gemm_tri(c, jb, m, jb, reinterpret_cast<const float*>(XL), jb, L21, lda, L21, lda, 1)))
@@ -1635,7 +1383,6 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
       const T* Yr = Y;
       int64_t ldyr = ldy;
       if (blocked) {
-        if (c->aux_stream) BEM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
         // TRSM of the block row in one product, Y = X U^{-1}
         float* X = reinterpret_cast<float*>(S + t0 + (int64_t)j0 * lda);
         const bool in_place = gemm_tri_in_place(c, m, jb, jb, X, lda);
@@ -1649,24 +1396,17 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
       } else {
       // TRSM of the block row, Y = X U^{-1} with U the unit upper triangle of the panel's
       // diagonal block, in 128-wide column blocks: X_b -= Y_{<b} U_{<b,b}, Y_b = X_b inv(U_bb)
-      if constexpr (sizeof(T) == 8) {  // the inverses of the panel's diagonal blocks, in one launch
-        inv_unit_upper_f64_kernel<<<(jb + kInvBlock - 1) / kInvBlock, kTriThreads, inv_smem, c->stream>>>(
-            S + j0 + (int64_t)j0 * lda, lda, jb, V);
-        BEM_LAUNCH_CHECK(c);
-      }
+      // (the inverses of all of the panel's diagonal blocks in one launch)
+      inv_unit_upper_kernel<T><<<(jb + kInvBlock - 1) / kInvBlock, kTriThreads, inv_smem, c->stream>>>(
+          S + j0 + (int64_t)j0 * lda, lda, jb, V);
+      BEM_LAUNCH_CHECK(c);
       for (int b0 = 0; b0 < jb; b0 += kInvBlock) {
         const int bb = std::min(kInvBlock, jb - b0);
-        T* Vb = sizeof(T) == 8 ? V + (size_t)b0 * kInvBlock : V;
+        const T* Vb = V + (size_t)b0 * kInvBlock;
         T* Xb = S + t0 + (int64_t)(j0 + b0) * lda;
         if (b0 > 0 &&
             (rc = gemm<T>(c, m, bb, b0, Y, ldy, S + j0 + (int64_t)(j0 + b0) * lda, lda, Xb, lda, 0)))
           return rc;
-        if constexpr (sizeof(T) == 4) {
-          inv_unit_upper_f32_kernel<<<1, kInvThreads, 2 * kInvBlock * kInvBlock * sizeof(float), c->stream>>>(
-              reinterpret_cast<const float*>(S + (j0 + b0) + (int64_t)(j0 + b0) * lda), lda, bb,
-              reinterpret_cast<float*>(V), kInvBlock);
-          BEM_LAUNCH_CHECK(c);
-        }
         if ((rc = gemm<T>(c, m, bb, bb, Xb, lda, Vb, kInvBlock, Y + (int64_t)b0 * ldy, ldy, 1))) return rc;
       }
       }
@@ -2010,9 +1750,9 @@ template <typename T>
 __global__ void __launch_bounds__(kTriThreads) diag_inv_kernel(const T* __restrict__ S, int64_t lda, int n,
                                                                double* __restrict__ Dinv) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* U = reinterpret_cast<double*>(smem_raw);  // [128][kTriPitch], the strict upper part
+  double* U = reinterpret_cast<double*>(smem_raw);  // [128][P], the strict upper part
   __shared__ double dg[kSolveBlock];
-  constexpr int NB = kSolveBlock, P = kTriPitch;
+  constexpr int NB = kSolveBlock, P = kTriPitch<double>;
   const int blk = blockIdx.x;
   const bool lower = blockIdx.y == 0;
   const int k0 = blk * NB, jb = min(NB, n - k0);
@@ -2037,7 +1777,7 @@ __global__ void __launch_bounds__(kTriThreads) diag_inv_kernel(const T* __restri
       else U[i + j * P] = v[u];
     }
   }
-  unit_upper_inverse(U, U + 128 * P);
+  unit_upper_inverse<double, kTriThreads>(U, U + 128 * P);
   // the upper inverse, or diag(D)^{-1} W^T
   for (int idx = tid; idx < NB * NB; idx += kTriThreads) {
     const int i = idx % NB, j = idx / NB;
@@ -2452,7 +2192,7 @@ int lu_prepare_inverses(bem_ctx* c, const T* S, int64_t lda, int n) {
     c->dinv.release();
     BEM_CUDA(c, c->dinv.alloc(need));
   }
-  const int smem = kTriDoubles * (int)sizeof(double);
+  const int smem = kTriElems<double> * (int)sizeof(double);
   static DeviceOnce attr;  // per instantiation and device
   if (attr.pending()) {
     BEM_CUDA(c, cudaFuncSetAttribute(diag_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));

@@ -33,8 +33,7 @@ struct LUWorkspace {
   unsigned* barrier;  // grid-barrier counter (zeroed before every panel launch)
   int* status;        // [0] error code, [1] info (zeroed at the start of a factorisation)
   void* inv;          // the 128 x 128 diagonal-block inverses of a panel (T)
-  void* finv;         // FP32 panels: the panel's two full triangle inverses (2 nb x nb)
-                      // and their assembly's scratch (nb x 128), else null
+  void* finv;         // FP32 panels: the panel's two full triangle inverses (2 nb x nb), else null
   void* ybuf;         // ldy x nb of T
   int64_t ldy;
   int gmax;           // most CTAs a panel launch may use
@@ -61,6 +60,13 @@ int lu_solve_ws(bem_ctx* c, const T* S, int64_t lda, int n, const int* perm, dou
 int panel_cluster_lines();
 int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status, int* moved);
 int panel_rows_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int q1, const int* moved);
+
+// XU, XL (jb x jb, leading dimension jb) := the inverses of the unit upper triangle and of the
+// lower triangle (diagonal included) of D (jb x jb, jb a multiple of 128, 16-byte aligned), zero
+// outside their triangles, in one cooperative launch (panel_inv.cu).  barrier, bar_base, status:
+// the factorisation's grid-barrier counter, its base so far (advanced) and error word.
+int panel_inverses_launch(bem_ctx* c, const float* D, int64_t lda, int jb, float* XU, float* XL, unsigned* barrier,
+                          unsigned& bar_base, int* status);
 
 template <typename T>
 int lu_factor(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int nb, int* info);

@@ -1,16 +1,34 @@
-// Inverse of a 128 x 128 unit upper triangle in shared memory, FP64, in place.
+// Inverse of a 128 x 128 unit upper triangle in shared memory, in place.
 #pragma once
 
 namespace bem {
 
-constexpr int kTriPitch = 130;    // column pitch: even, so that four rows of a column load as two 16 B words
-constexpr int kTriThreads = 512;  // threads of a CTA that inverts
+// column pitch: four rows of a column load as 16-byte words
+template <typename T>
+constexpr int kTriPitch = sizeof(T) == 8 ? 130 : 132;
+constexpr int kTriThreads = 512;  // threads of a CTA that only inverts
 // shared memory of unit_upper_inverse: the triangle and a 96 x 32 product
-constexpr int kTriDoubles = 128 * kTriPitch + 96 * 32;
+template <typename T>
+constexpr int kTriElems = 128 * kTriPitch<T> + 96 * 32;
+
+__device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = b.x;
+  v[3] = b.y;
+}
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x;
+  v[1] = a.y;
+  v[2] = a.z;
+  v[3] = a.w;
+}
 
 // U (column-major, pitch kTriPitch, 16-byte aligned; its strict upper part given, zero below
-// the diagonal, the diagonal itself ignored) := (I + strict upper part)^{-1}; all kTriThreads
-// threads take part, with a barrier before and after.
+// the diagonal, the diagonal itself ignored) := (I + strict upper part)^{-1}; all NT threads
+// of the CTA take part, with a barrier before and after.
 //
 // Blocked by 32 as LAPACK's dtrtri: four warps invert the diagonal blocks (a lane per column
 // in registers, column by column of U so that a step's updates are independent of each
@@ -18,16 +36,17 @@ constexpr int kTriDoubles = 128 * kTriPitch + 96 * 32;
 //   V_{<j,j} = -V_{<j,<j} (U_{<j,j} V_jj),
 // two products per block column, four rows and one column per thread and step, everything
 // in shared memory.  (Kept in global memory and taken block by block, 18 barriers and an L2
-// round trip per product, the same inverse took 97 us; a 128-block now takes 20 us.)
-__device__ __forceinline__ void unit_upper_inverse(double* U, double* T) {
-  constexpr int B = 32, P = kTriPitch;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kTriThreads / 32;
+// round trip per product, the FP64 inverse took 97 us; a 128-block now takes 20 us.)
+template <typename T, int NT>
+__device__ __forceinline__ void unit_upper_inverse(T* U, T* W) {
+  constexpr int B = 32, P = kTriPitch<T>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = NT / 32;
   __syncthreads();
   if (warp < 4) {
-    double* D = U + warp * B * (P + 1);
-    double x[B];
+    T* D = U + warp * B * (P + 1);
+    T x[B];
 #pragma unroll
-    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? 1.0 : 0.0;
+    for (int i = 0; i < B; ++i) x[i] = (i == lane) ? T(1) : T(0);
 #pragma unroll
     for (int k = B - 1; k > 0; --k)
 #pragma unroll
@@ -40,42 +59,33 @@ __device__ __forceinline__ void unit_upper_inverse(double* U, double* T) {
   __syncthreads();
   for (int j = 1; j < 4; ++j) {
     const int R = B * j;
-    // T (R x 32, [k][row pairs] as T[row + 96 c]) = U_{<j,j} V_jj
+    // W (R x 32, row by row) = U_{<j,j} V_jj
     for (int g = warp; g < R / 4; g += nw) {
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      T s[4] = {};
 #pragma unroll 8
       for (int k = 0; k < B; ++k) {
-        const double2* a = reinterpret_cast<const double2*>(U + 4 * g + (R + k) * P);
-        const double2 a0 = a[0], a1 = a[1];
-        const double b = U[R + k + (R + lane) * P];  // zero below V_jj's diagonal
-        s0 = fma(a0.x, b, s0);
-        s1 = fma(a0.y, b, s1);
-        s2 = fma(a1.x, b, s2);
-        s3 = fma(a1.y, b, s3);
+        T a[4];
+        load4(U + 4 * g + (R + k) * P, a);
+        const T b = U[R + k + (R + lane) * P];  // zero below V_jj's diagonal
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] = fma(a[i], b, s[i]);
       }
-      T[(4 * g + 0) * B + lane] = s0;
-      T[(4 * g + 1) * B + lane] = s1;
-      T[(4 * g + 2) * B + lane] = s2;
-      T[(4 * g + 3) * B + lane] = s3;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) W[(4 * g + i) * B + lane] = s[i];
     }
     __syncthreads();
     for (int g = warp; g < R / 4; g += nw) {
-      double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+      T s[4] = {};
 #pragma unroll 4
       for (int k = 4 * g; k < R; ++k) {
-        const double2* a = reinterpret_cast<const double2*>(U + 4 * g + k * P);
-        const double2 a0 = a[0], a1 = a[1];
-        const double b = T[k * B + lane];
-        s0 = fma(a0.x, b, s0);
-        s1 = fma(a0.y, b, s1);
-        s2 = fma(a1.x, b, s2);
-        s3 = fma(a1.y, b, s3);
+        T a[4];
+        load4(U + 4 * g + k * P, a);
+        const T b = W[k * B + lane];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s[i] = fma(a[i], b, s[i]);
       }
-      double* o = U + 4 * g + (R + lane) * P;  // the columns of block j are not read here
-      o[0] = -s0;
-      o[1] = -s1;
-      o[2] = -s2;
-      o[3] = -s3;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) U[4 * g + i + (R + lane) * P] = -s[i];  // not read by this product
     }
     __syncthreads();
   }

@@ -264,75 +264,126 @@ __device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, in
   }
 }
 
-// window_lu_warp for a full FP32 window with lane c's column in registers, shifted so
-// that every index is static: at step t, v[k] holds row t + k of the lane's column, and
-// row t's final value (the pivot row's entry, or the multiplier) is stored to D[lane][t]
-// before the shift.  The pivot column is broadcast by shuffles; an interchange moves
-// the two lanes' registers (and their original indices) by shuffles and the rows
-// already stored by one swap per lane.  The pivot rule (largest magnitude among lanes
-// >= t, ties to the smallest index, after a vote on whether any lane beats the
-// diagonal) and the arithmetic (one IEEE division per multiplier, one fused
-// multiply-add per entry) are window_lu_warp's, and so are the results, bit for bit.
-// s_p[t] receives step t's local pivot; s_g[b] the original window column of factored
-// column b.  (Measured on one warp: 14,000 cycles for a diagonally dominant window,
-// against 22,700 for window_lu_warp.)
-__device__ __forceinline__ void window_lu_warp_f32(float (*D)[kPanelW + 1], int* s_p, int* s_g, int lane) {
-  constexpr int W = kPanelW;
+// LU with partial pivoting of a full FP32 32 x 32 window by eight warps: lane c of warp g holds
+// rows 4 g .. 4 g + 3 of window column c, loaded by load(c, row) as one 16-byte word.  Warp g
+// takes the four steps of its rows by itself (a vote and a few shuffles each), then publishes
+// their multipliers and pivot lanes, and the warps below apply the four rank-1 updates: one CTA
+// barrier per four steps.  A column never moves: its lane keeps the position that the
+// interchanges give it (as in panel_cluster.cuh).  The pivot rule is window_lu_warp's (largest
+// magnitude among positions >= t, ties to the smallest one, NaN never chosen); a multiplier is
+// the product with the pivot's reciprocal corrected by its remainder, an entry one fused
+// multiply-add per step.  What bounds it is the chain of 32 pivots (vote, shuffle, reciprocal:
+// 210 cycles each), and after each barrier the four updates of the next warp (400 cycles).
+// On return (after a barrier) D[b][j] holds row j of the factored column at position b, s_p[t]
+// step t's local pivot, s_g[b] the original column of position b.  All threads of the CTA call
+// it; the warps past the eighth keep the barriers only.  (One warp with a column per lane and
+// the pivot column by 31 shuffles a step took 14,000 cycles for a diagonally dominant window,
+// this 10,000; a branch around the updates of a warp costs 300 cycles a group.)
+__device__ __forceinline__ float reciprocal_f32(float x) {  // the approximation and one Newton step
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(y, fmaf(-x, y, 1.f), y);
+}
+// kept out of line: as a select it would be computed for every multiplier
+__device__ __noinline__ float window_quotient(float a, float b) { return a / b; }
+
+struct WindowScratch {  // by parity of the group
+  float4 l[2][kPanelW];  // a column's multipliers of the four steps (0: no update)
+  int4 lane[2];          // the pivots' lanes
+  int4 from[2];          // and positions before their interchanges
+};
+template <typename Load>
+__device__ __forceinline__ void window_lu_cta(WindowScratch& ws, float (*D)[kPanelW + 1], int* s_p, int* s_g,
+                                              Load load) {
+  constexpr int W = kPanelW, G = W / 4;
   constexpr unsigned FULL = 0xffffffffu;
-  float v[W];
-#pragma unroll
-  for (int j = 0; j < W; ++j) v[j] = D[lane][j];
-  int g = lane;
-#pragma unroll 1
-  for (int t = 0; t < W; ++t) {
-    float ct = v[0];
-    float pv = __shfl_sync(FULL, ct, t);
-    int p = t;
-    if (__any_sync(FULL, lane > t && fabsf(ct) > fabsf(pv))) {
-      float bv = (lane >= t) ? fabsf(ct) : -1.f;
-      int bc = (lane >= t) ? lane : INT_MAX;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float ov = __shfl_xor_sync(FULL, bv, off);
-        const int oc = __shfl_xor_sync(FULL, bc, off);
-        if (ov > bv || (ov == bv && oc < bc)) {
-          bv = ov;
-          bc = oc;
-        }
-      }
-      p = bc;
-      if (p != t) {  // lanes t and p exchange their columns
-        const int src = (lane == t) ? p : ((lane == p) ? t : lane);
-#pragma unroll
-        for (int j = 0; j < W; ++j) v[j] = __shfl_sync(FULL, v[j], src);
-        g = __shfl_sync(FULL, g, src);
-        if (lane < t) {  // the rows already stored: lane j swaps its row j
-          const float a = D[t][lane];
-          D[t][lane] = D[p][lane];
-          D[p][lane] = a;
-        }
-        ct = v[0];
-        pv = __shfl_sync(FULL, ct, t);
-      }
-    }
-    if (lane == 0) s_p[t] = p;
-    float pr[W];
-#pragma unroll
-    for (int k = 1; k < W; ++k) pr[k] = __shfl_sync(FULL, v[k], t);
-    if (pv != 0.f && lane > t) {
-      const float l = ct / pv;
-#pragma unroll
-      for (int k = 1; k < W; ++k) v[k] -= l * pr[k];
-      v[0] = l;
-    }
-    D[lane][t] = v[0];
-#pragma unroll
-    for (int k = 0; k < W - 1; ++k) v[k] = v[k + 1];
-    v[W - 1] = 0.f;
-    __syncwarp();
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (g < G) {
+    const float4 x = load(lane, 4 * g);
+    v[0] = x.x;
+    v[1] = x.y;
+    v[2] = x.z;
+    v[3] = x.w;
   }
-  s_g[lane] = g;
-  __syncwarp();
+  int pos = lane;
+  bool moved = false;  // an interchange so far (the same in all lanes)
+#pragma unroll 1
+  for (int k = 0; k < G; ++k) {
+    const int par = k & 1;
+    if (g == k) {
+      float lv[4];
+      int pls[4], frs[4];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int t = 4 * k + s;
+        const float ct = v[s];
+        int pl = moved ? __ffs(__ballot_sync(FULL, pos == t)) - 1 : t;  // the lane at position t
+        float pv = __shfl_sync(FULL, ct, pl), u[4];
+#pragma unroll
+        for (int i = s + 1; i < 4; ++i) u[i] = __shfl_sync(FULL, v[i], pl);
+        int from = t;
+        if (__any_sync(FULL, pos > t && fabsf(ct) > fabsf(pv))) {
+          const unsigned key = (pos >= t && ct == ct) ? __float_as_uint(fabsf(ct)) : 0u;
+          const unsigned most = __reduce_max_sync(FULL, key);
+          from = (int)__reduce_min_sync(FULL, pos >= t && key == most ? (unsigned)pos : (unsigned)W);
+          const int old = pl;
+          pl = __ffs(__ballot_sync(FULL, pos == from)) - 1;
+          if (lane == old) pos = from;
+          if (lane == pl) pos = t;
+          moved = true;
+          pv = __shfl_sync(FULL, ct, pl);
+#pragma unroll
+          for (int i = s + 1; i < 4; ++i) u[i] = __shfl_sync(FULL, v[i], pl);
+        }
+        const float rp = reciprocal_f32(pv);
+        float l = ct * rp;
+        l = fmaf(fmaf(-l, pv, ct), rp, l);
+        if (!(fabsf(pv) > 1e-30f && fabsf(pv) < 1e30f)) l = window_quotient(ct, pv);  // near the range's ends
+        const bool upd = pos > t && pv != 0.f;
+        lv[s] = upd ? l : 0.f;
+        v[s] = upd ? l : ct;
+#pragma unroll
+        for (int i = s + 1; i < 4; ++i) v[i] = upd ? fmaf(-l, u[i], v[i]) : v[i];
+        pls[s] = pl;
+        frs[s] = from;
+      }
+      ws.l[par][lane] = make_float4(lv[0], lv[1], lv[2], lv[3]);
+      if (lane == 0) {
+        ws.lane[par] = make_int4(pls[0], pls[1], pls[2], pls[3]);
+        ws.from[par] = make_int4(frs[0], frs[1], frs[2], frs[3]);
+        *reinterpret_cast<int4*>(s_p + 4 * k) = make_int4(frs[0], frs[1], frs[2], frs[3]);
+      }
+    }
+    __syncthreads();
+    // without branches (a branch the compiler cannot prove uniform costs a convergence barrier
+    // around every shuffle): the warps above and the owner apply zeros, the owner no interchange
+    {
+      float4 l4 = ws.l[par][lane];
+      const int4 p4 = ws.lane[par], f4 = ws.from[par];
+      const float lq[4] = {l4.x, l4.y, l4.z, l4.w};
+      const int pl[4] = {p4.x, p4.y, p4.z, p4.w}, fr[4] = {f4.x, f4.y, f4.z, f4.w};
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        const int t = 4 * k + s, from = g == k ? t : fr[s];
+        pos = pos == t ? from : pos;
+        pos = lane == pl[s] ? t : pos;
+        moved |= fr[s] != t;
+        const float l = g > k ? lq[s] : 0.f;
+        float u[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) u[i] = __shfl_sync(FULL, v[i], pl[s]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = l != 0.f ? fmaf(-l, u[i], v[i]) : v[i];
+      }
+    }
+  }
+  if (g < G) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) D[pos][4 * g + i] = v[i];
+    if (g == 0) s_g[pos] = lane;
+  }
+  __syncthreads();
 }
 
 // Window pivoting: the sub-panel's pivot search is restricted to its w x w diagonal
@@ -456,8 +507,7 @@ __global__ void __launch_bounds__(256) window_panel_kernel(T* S, int64_t lda, in
 
 // The whole step of one 32-wide sub-panel of a window-pivoted FP32 panel in one CTA
 // (the panel's diagonal block only; rows and columns outside it follow per panel):
-// warp 0 factors the 32 x 32 window in registers while the other threads load their
-// columns; every thread then eliminates its column of the sub-panel (columns
+// the 32 x 32 window is factored in registers; every thread then eliminates its column of the sub-panel (columns
 // [r0 + 32, t0)), the factored window goes back into S, and one thread per row of the
 // block applies the window's interchanges as a gather and, below the window, the
 // unit-lower TRSM of trsm_small_kernel.  Pivots and the first exact zero pivot as
@@ -467,7 +517,8 @@ __global__ void __launch_bounds__(kBlockThreads) window_block_kernel(float* S, i
                                                                      int* piv, int* status) {
   constexpr int W = kPanelW;
   __shared__ float D[W][W + 1];  // D[c][j] = S(r0 + j, r0 + c)
-  __shared__ int s_p[W], s_g[W];
+  __shared__ __align__(16) int s_p[W], s_g[W];
+  __shared__ WindowScratch s_w;
   const int tid = threadIdx.x, lane = tid & 31;
   const int c = r0 + W + tid;  // this thread's column
   float x[W];
@@ -483,11 +534,10 @@ __global__ void __launch_bounds__(kBlockThreads) window_block_kernel(float* S, i
       x[4 * q + 3] = v.w;
     }
   }
+  window_lu_cta(s_w, D, s_p, s_g, [&](int cc, int j) {  // s_g: the interchanges as a gather, y[b] = x[s_g[b]]
+    return *reinterpret_cast<const float4*>(S + r0 + j + (int64_t)(r0 + cc) * lda);
+  });
   if (tid < W) {
-#pragma unroll
-    for (int cc = 0; cc < W; ++cc) D[cc][lane] = S[r0 + lane + (int64_t)(r0 + cc) * lda];
-    __syncwarp();
-    window_lu_warp_f32(D, s_p, s_g, lane);  // s_g: the interchanges as a gather, y[b] = x[s_g[b]]
     if (lane == 0) {
       for (int t = 0; t < W; ++t)
         if (D[t][t] == 0.f) {
@@ -543,9 +593,8 @@ __global__ void __launch_bounds__(kBlockThreads) window_block_kernel(float* S, i
 // The diagonal block [j0, t0)^2 of a window-pivoted FP32 panel in one cooperative
 // launch: the 32-wide sub-panels in turn, each in three phases separated by grid
 // barriers (two per sub-panel) instead of kernel boundaries:
-//   A  every CTA's warp 0 stages and factors the 32 x 32 window (redundantly; the
-//      interchanges composed into a gather on the way); CTA 0 records the pivots and
-//      the first exact zero pivot;
+//   A  every CTA factors the 32 x 32 window (redundantly; the interchanges composed into a
+//      gather on the way); CTA 0 records the pivots and the first exact zero pivot;
 //   B  the sub-panel's vectors, one thread each, spread over the CTAs in contiguous
 //      runs: every column c in [r0 + 32, t0) eliminated with the window's steps
 //      (window_panel_kernel's column operations, with each multiplier formed by the
@@ -568,7 +617,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   constexpr int TP = kCoopTile + 4;  // strip pitch: 16-byte rows, 4-way store conflicts at most
   __shared__ float D[W][W + 1];     // D[c][j] = S(r0 + j, r0 + c)
   __shared__ float rdg[W];          // reciprocal pivots (0 for an exact zero pivot)
-  __shared__ int s_p[W], s_g[W];
+  __shared__ WindowScratch s_w;
+  __shared__ __align__(16) int s_p[W], s_g[W];
   __shared__ __align__(16) float Ls[W][TP];  // Ls[k][r] = S(q0 + tr + r, r0 + k)
   __shared__ __align__(16) float Us[W][TP];  // Us[k][c] = S(r0 + k, q0 + tc + c)
   __shared__ int s_abort;
@@ -577,24 +627,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   for (int r0 = j0; r0 < t0; r0 += W) {
     const int q0 = r0 + W, m = t0 - q0;
     // A: the window
+    window_lu_cta(s_w, D, s_p, s_g, [&](int cc, int j) {
+      return __ldcg(reinterpret_cast<const float4*>(S + r0 + j + (int64_t)(r0 + cc) * lda));
+    });
     if (tid < W) {
-      float wv[W];  // every load in flight before the first store
-#pragma unroll
-      for (int cc = 0; cc < W; ++cc) wv[cc] = __ldcg(S + r0 + lane + (int64_t)(r0 + cc) * lda);
-#pragma unroll
-      for (int cc = 0; cc < W; ++cc) D[cc][lane] = wv[cc];
-      __syncwarp();
-      window_lu_warp_f32(D, s_p, s_g, lane);
-      rdg[lane] = (D[lane][lane] != 0.f) ? __frcp_rn(D[lane][lane]) : 0.f;
+      const float d = D[lane][lane];
+      rdg[lane] = (d != 0.f) ? __frcp_rn(d) : 0.f;
       if (g == 0) {
         piv[r0 + lane] = r0 + s_p[lane];
-        if (lane == 0) {
-          for (int t = 0; t < W; ++t)
-            if (D[t][t] == 0.f) {
-              if (status[1] == 0) status[1] = r0 + t + 1;
-              break;
-            }
-        }
+        const unsigned zero = __ballot_sync(0xffffffffu, d == 0.f);
+        if (lane == 0 && zero != 0 && status[1] == 0) status[1] = r0 + __ffs(zero);
       }
     }
     __syncthreads();

@@ -14,6 +14,8 @@
 //                       and to the trailing rows (contiguous column segments)
 //     trsm_small + gemm update of the panel rows below the sub-panel
 //   inv_unit_upper + gemm (TRSM by inverse), then the trailing gemm update.
+#include <cuda.h>
+
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -990,6 +992,9 @@ int gemm_bf16(bem_ctx* c, int M, int N, int K, const float* A, int64_t lda, cons
               int64_t ldc, int mode, int split);
 bool gemm_tc_ok(const void* A, int64_t lda, const void* B, int64_t ldb, int elem);
 bool umma_supported(int K);
+// The tensor map of a column-major FP32 matrix in boxes of box_rows x box_cols, zeros past its edges.
+int tma_map_f32(bem_ctx* c, CUtensorMap* map, const float* A, int rows, int cols, int64_t ld, int box_rows,
+                int box_cols);
 int umma_reserve(bem_ctx* c, int M, int N, int K);
 int gemm_umma_bf16(bem_ctx* c, int M, int N, int K, const float* A, int64_t lda, const float* B, int64_t ldb,
                    float* C, int64_t ldc, int nprod, bool store, int kmode);
@@ -1841,7 +1846,31 @@ __device__ __forceinline__ void ld_volatile_v2(const unsigned long long* p, unsi
   asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }
 
-// One sweep over the 128-row blocks with the diagonal blocks' inverses.  UPPER as in
+__device__ __forceinline__ void publish_word(unsigned long long* p, unsigned tag, double x) {
+  const unsigned long long hi = (unsigned long long)tag << 32;
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
+  st_volatile_v2(p, hi | (bits & 0xffffffffull), hi | (bits >> 32));
+}
+
+// waits for the two words of an unknown; 0 with *status and *abort set when the wait runs out
+__device__ __forceinline__ double poll_word(const unsigned long long* p, unsigned tag, int* status,
+                                            unsigned long long wait_ns, int* abort) {
+  const unsigned long long t0 = globaltimer_ns();
+  unsigned it = 0;
+  unsigned long long w0, w1;
+  for (;;) {
+    ld_volatile_v2(p, w0, w1);
+    if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag) break;
+    if ((++it & 63u) == 0 && (globaltimer_ns() - t0 > wait_ns || *((volatile int*)status) != 0)) {
+      atomicCAS(status, 0, BEM_ERR_TIMEOUT);
+      *abort = 1;
+      return 0.0;
+    }
+  }
+  return __longlong_as_double((long long)((w1 << 32) | (w0 & 0xffffffffull)));
+}
+
+// One sweep over the 128-row blocks of FP64 factors with the diagonal blocks' inverses.  UPPER as in
 // sweep_kernel.  Step s solves block k(s) and is owned by CTA s % G, which keeps the
 // partial right-hand sides w of its blocks in shared memory (w = b - the tiles of the
 // blocks solved so far).  A solved block is published as 256 words {tag, 32 data bits}
@@ -1852,14 +1881,13 @@ __device__ __forceinline__ void ld_volatile_v2(const unsigned long long* p, unsi
 // A wait that exceeds the context's wait limit records BEM_ERR_TIMEOUT in *status and
 // ends the CTA.  `withhold` (failure injection, -1 = none) is a step of the forward
 // sweep that is solved but not published, so that the waits for it run out.
-template <typename T, bool UPPER>
+template <bool UPPER>
 __global__ void __launch_bounds__(kSweepThreads, 1)
-    sweep_inv_kernel(const T* __restrict__ S, int64_t lda, int n, const double* __restrict__ Dinv, double* b,
+    sweep_inv_kernel(const double* __restrict__ S, int64_t lda, int n, const double* __restrict__ Dinv, double* b,
                      unsigned long long* slots, unsigned tag, int* status, unsigned long long wait_ns,
                      int withhold) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NB = kSolveBlock;
-  constexpr bool kPrefetch = sizeof(T) == 4;  // double-buffered tile registers for FP32 factors
   double* Di = reinterpret_cast<double*>(smem_raw);  // [NB * NB] inverse of the next owned block
   double* wacc = Di + NB * NB;                        // [owned blocks][NB]
   __shared__ double ys[NB];
@@ -1880,12 +1908,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
       for (int u = 0; u < 8; ++u) dst[i0 + u * kSweepThreads + t] = v[u];
     }
   };
-  auto load_tile = [&](T* a, int sx, int c0, int cb) {
+  auto load_tile = [&](double* a, int sx, int c0, int cb) {
     const int r0 = bidx(sx) * NB, rb = min(NB, n - r0);
     const int cq = 32 * q;
-    const T* p = S + (r0 + rl) + (int64_t)(c0 + cq) * lda;
+    const double* p = S + (r0 + rl) + (int64_t)(c0 + cq) * lda;
 #pragma unroll
-    for (int u = 0; u < 32; ++u) a[u] = (rl < rb && cq + u < cb) ? p[(int64_t)u * lda] : T(0);
+    for (int u = 0; u < 32; ++u) a[u] = (rl < rb && cq + u < cb) ? p[(int64_t)u * lda] : 0.0;
   };
   const int nown = (g < nblk) ? (nblk - 1 - g) / G + 1 : 0;
   for (int i = t; i < nown * NB; i += blockDim.x) {
@@ -1906,10 +1934,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     __syncthreads();
     if (t < kb) {
       const double x = (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
-      const unsigned long long hi = (unsigned long long)tag << 32;
-      const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
       if (UPPER || s != withhold)  // a withheld step (failure injection) is never published
-        st_volatile_v2(slots + (size_t)s * 256 + 2 * t, hi | (bits & 0xffffffffull), hi | (bits >> 32));
+        publish_word(slots + (size_t)s * 256 + 2 * t, tag, x);
       b[k0 + t] = x;
     }
     __syncthreads();  // Di and red are free again
@@ -1921,54 +1947,310 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     const int s2 = s + 1 + ((g - (s + 1)) % G + G) % G;  // this CTA's first step after s
     if (s2 >= nblk) break;                                // no rows left to update
     const int c0 = bidx(s) * NB, cb = min(NB, n - c0);
-    T a[32];
+    double a[32];
     load_tile(a, s2, c0, cb);
-    if (t < NB) {
-      double y = 0.0;
-      if (t < cb) {
-        const unsigned long long* p = slots + (size_t)s * 256 + 2 * t;
-        const unsigned long long t0 = globaltimer_ns();
-        unsigned it = 0;
-        unsigned long long w0, w1;
-        for (;;) {
-          ld_volatile_v2(p, w0, w1);
-          if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag) break;
-          if ((++it & 63u) == 0 &&
-              (globaltimer_ns() - t0 > wait_ns || *((volatile int*)status) != 0)) {
-            atomicCAS(status, 0, BEM_ERR_TIMEOUT);
-            s_abort = 1;
-            w0 = w1 = 0;
-            break;
-          }
-        }
-        y = __longlong_as_double((long long)((w1 << 32) | (w0 & 0xffffffffull)));
-      }
-      ys[t] = y;
-    }
+    if (t < NB) ys[t] = t < cb ? poll_word(slots + (size_t)s * 256 + 2 * t, tag, status, wait_ns, &s_abort) : 0.0;
     __syncthreads();
     if (s_abort) return;
     for (int sx = s2; sx < nblk; sx += G) {
-      const bool more = sx + G < nblk;
-      T nx[32];
-      if (kPrefetch && more) load_tile(nx, sx + G, c0, cb);
       double acc = 0.0;
 #pragma unroll
-      for (int u = 0; u < 32; ++u) acc = fma((double)a[u], ys[32 * q + u], acc);
+      for (int u = 0; u < 32; ++u) acc = fma(a[u], ys[32 * q + u], acc);
       red[q][rl] = acc;
       __syncthreads();
       if (t < NB) wacc[((sx - g) / G) * NB + t] -= (red[0][t] + red[1][t]) + (red[2][t] + red[3][t]);
       __syncthreads();
       if (sx == s + 1) solve(sx);
-      if (more) {
-        if (kPrefetch) {
-#pragma unroll
-          for (int u = 0; u < 32; ++u) a[u] = nx[u];
-        } else {
-          load_tile(a, sx + G, c0, cb);
-        }
-      }
+      if (sx + G < nblk) load_tile(a, sx + G, c0, cb);
     }
   }
+}
+
+// ---- the sweeps of FP32 factors ----------------------------------------------------------
+// lead[2 blk] = (inverse of blk's lower triangle) S(blk, blk - 1) and lead[2 blk + 1] = (inverse
+// of its upper triangle) S(blk, blk + 1), each 128 x 128, column-major, FP64: the block's solution
+// is Dinv w - lead y with y the block solved just before and w free of it, so Dinv w is formed
+// while y is still on its way.  Grid (blocks, 2); bound by the FP64 pipe (128^3 multiply-adds a
+// CTA), once per factorisation.
+constexpr int kLeadThreads = 256, kLeadK = 32, kLeadP = kSolveBlock + 1;
+__global__ void __launch_bounds__(kLeadThreads) lead_kernel(const float* __restrict__ S, int64_t lda, int n,
+                                                            const double* __restrict__ Dinv,
+                                                            double* __restrict__ lead) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NB = kSolveBlock;
+  double* As = reinterpret_cast<double*>(smem_raw);  // [kLeadK][NB] columns of the inverse
+  double* Bs = As + kLeadK * NB;                      // [kLeadK][kLeadP] rows of S's block
+  const int blk = blockIdx.x, nblk = gridDim.x, side = blockIdx.y, nb = side ? blk + 1 : blk - 1;
+  if (nb < 0 || nb >= nblk) return;  // the first step's block has none
+  const int r0 = blk * NB, c0 = nb * NB, rb = min(NB, n - r0), cb = min(NB, n - c0);
+  const double* V = Dinv + ((size_t)blk * 2 + side) * (NB * NB);
+  const float* B = S + r0 + (int64_t)c0 * lda;
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
+  double acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
+  for (int k0 = 0; k0 < NB; k0 += kLeadK) {
+#pragma unroll
+    for (int u = 0; u < kLeadK * NB / kLeadThreads; ++u) {
+      const int idx = t + u * kLeadThreads;
+      As[idx] = V[k0 * NB + idx];
+      const int kk = idx % kLeadK, j = idx / kLeadK;
+      Bs[kk * kLeadP + j] = k0 + kk < rb && j < cb ? (double)B[k0 + kk + (int64_t)j * lda] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int kk = 0; kk < kLeadK; ++kk) {
+      double a[8], b[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = As[kk * NB + ty + 16 * i];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) b[j] = Bs[kk * kLeadP + tx + 16 * j];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+    }
+    __syncthreads();
+  }
+  // through shared memory, so that a column leaves as whole sectors
+  double* out = lead + ((size_t)blk * 2 + side) * (NB * NB);
+#pragma unroll
+  for (int jj = 0; jj < 8; ++jj) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) As[tx * kLeadP + ty + 16 * i] = acc[i][jj];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 16 * NB / kLeadThreads; ++u) {
+      const int idx = t + u * kLeadThreads, r = idx % NB, j = idx / NB;
+      out[r + (j + 16 * jj) * NB] = As[j * kLeadP + r];
+    }
+    __syncthreads();
+  }
+}
+constexpr int kLeadSmem = (kLeadK * kSolveBlock + kLeadK * kLeadP) * (int)sizeof(double);
+static_assert(16 * kLeadP <= kLeadK * kSolveBlock, "the staged columns fit in As");
+
+__device__ __forceinline__ void cp_async_16(unsigned dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__device__ __forceinline__ void tile_bar_init(unsigned bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+}
+// a box of a tensor map to shared memory; `bar` completes its phase when all bytes are there
+__device__ __forceinline__ void tile_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar, int bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ bool tile_ready(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+__device__ __forceinline__ bool tile_wait(unsigned bar, unsigned parity, unsigned long long wait_ns) {
+  if (tile_ready(bar, parity)) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  while (!tile_ready(bar, parity))
+    if (globaltimer_ns() - t0 > wait_ns) return false;
+  return true;
+}
+
+// sweep_inv_kernel's schedule, slots and waits for FP32 factors.  Two things bound it: the tiles
+// (64 KB each, every one read once) and the chain of publications.
+// * A ring of two tiles in shared memory is filled by the Tensor Memory Accelerator across the
+//   steps' borders, so that the loads never stop at a wait for a block.
+// * The owner of step s + 1 forms z = Dinv w before y_s arrives, from the inverse staged in shared
+//   memory one owned step ahead, and x = z - lead y_s is one 128 x 128 FP64 product from
+//   registers, loaded an owned step ahead too: an SM reads 64 bytes a cycle from L2, 1.1 us for
+//   either block.  Publication to publication: one poll, 32 multiply-adds and two barriers.
+// One CTA barrier per tile: the partial sums alternate between two buffers.  A tile costs 1,024
+// cycles of conversions to FP64 (a quarter of the multiply-add's rate).
+// Measured, a sweep of 56,000 unknowns: 1.29 ms (4.9 TB/s), of 18,432: 0.28 ms (1.9 us a block);
+// with tiles two deep in registers and inverse and product between poll and publication 2.36 and
+// 0.41 ms.  Loading the lead block or the inverse when it is needed costs 1 us a block each;
+// 16-byte copies by the threads instead of TMA boxes 1.7 us a tile.
+constexpr int kSweepTileBytes = kSolveBlock * kSolveBlock * (int)sizeof(float);
+constexpr int kSweepInvSmem = 10 * 32 * 32 * (int)sizeof(double);  // a triangle's 32 x 32 blocks
+template <bool UPPER>
+__global__ void __launch_bounds__(kSweepThreads, 1)
+    sweep_ring_kernel(const __grid_constant__ CUtensorMap map, int n, const double* __restrict__ Dinv,
+                      const double* __restrict__ lead, double* b, unsigned long long* slots, unsigned tag,
+                      int* status, unsigned long long wait_ns, int withhold) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int NB = kSolveBlock;
+  // a box lands on a 128-byte boundary (the launch adds the room)
+  unsigned char* smem = smem_raw + (-(unsigned)__cvta_generic_to_shared(smem_raw) & 127u);
+  // [2 tiles][column][row]; [10 blocks][column][row], the next owned block's inverse;
+  // [owned blocks][NB]
+  float* ring = reinterpret_cast<float*>(smem);
+  double* wacc = reinterpret_cast<double*>(smem + 2 * kSweepTileBytes + kSweepInvSmem);
+  __shared__ __align__(16) double ys[NB];
+  __shared__ double red[2][4][NB];
+  __shared__ __align__(8) unsigned long long s_bar[2];
+  __shared__ int s_abort;
+  const int t = threadIdx.x, lane = t & 31, G = gridDim.x, g = blockIdx.x;
+  const int nblk = (n + NB - 1) / NB;
+  const int rl = t & (NB - 1), q = t >> 7;  // this thread's row; its columns are 32 q .. 32 q + 31
+  const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
+  const unsigned bar_s = (unsigned)__cvta_generic_to_shared(s_bar);
+  // this warp's 32 x 32 block (row block rq, column block q) of the inverse, if not zero
+  const int rq = rl >> 5, hi = max(rq, q), lo = min(rq, q);
+  const bool inv_mine = UPPER ? rq <= q : rq >= q;
+  double* Di = reinterpret_cast<double*>(smem + 2 * kSweepTileBytes) + (hi * (hi + 1) / 2 + lo) * 1024;
+  auto bidx = [&](int s) { return UPPER ? nblk - 1 - s : s; };
+  auto first = [&](int s) { return s + 1 + ((g - (s + 1)) % G + G) % G; };  // this CTA's first step after s
+  auto block = [&](const double* base, int s) { return base + ((size_t)bidx(s) * 2 + (UPPER ? 1 : 0)) * (NB * NB); };
+
+  // thread 0: the tiles in the order of their use, all but each step's lead block
+  int fs = 0, fx = nblk > 1 ? first(0) : nblk, asked = 0;
+  auto fill = [&]() {
+    for (;;) {  // past a lead block, past a step's last tile
+      if (fx >= nblk) {
+        if (++fs + 1 >= nblk || (fx = first(fs)) >= nblk) {  // no rows left in this or any later step
+          fs = fx = nblk;
+          return;
+        }
+      } else if (fx == fs + 1) {
+        fx += G;
+      } else {
+        break;
+      }
+    }
+    const int h = asked & 1;
+    tile_load(ring_s + h * kSweepTileBytes, &map, bidx(fx) * NB, bidx(fs) * NB, bar_s + 8 * h, kSweepTileBytes);
+    ++asked;
+    fx += G;
+  };
+  // the inverse and the lead block of an owned step
+  double m[32];
+  auto stage = [&](int s) {
+    if (inv_mine) {
+      const double* D = block(Dinv, s) + 32 * rq + 32 * q * NB + 2 * (lane & 15) + (lane >> 4) * NB;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(Di) + lane * 16;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) cp_async_16(dst + u * 512, D + 2 * u * NB);
+    }
+    if (s > 0) {
+      const double* M = block(lead, s) + rl + 32 * q * NB;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) m[u] = __ldcg(M + u * NB);
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < 32; ++u) m[u] = 0.0;
+  if (t == 0) {
+    tile_bar_init(bar_s);
+    tile_bar_init(bar_s + 8);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    s_abort = 0;
+    fill();
+    fill();
+  }
+  if (g < nblk) stage(g);
+  const int nown = (g < nblk) ? (nblk - 1 - g) / G + 1 : 0;
+  for (int i = t; i < nown * NB; i += blockDim.x) {
+    const int k0 = bidx(g + (i / NB) * G) * NB, r = i % NB;
+    wacc[i] = (k0 + r < n) ? b[k0 + r] : 0.0;
+  }
+  cp_async_all();
+  __syncthreads();
+
+  auto inv_product = [&](int s) {  // this thread's share of Dinv w for step s
+    const double* D = Di + lane;
+    const double2* wo = reinterpret_cast<const double2*>(wacc + ((s - g) / G) * NB + 32 * q);
+    double acc = 0.0;
+    if (inv_mine) {
+#pragma unroll 8
+      for (int u = 0; u < 16; ++u) {
+        const double2 x = wo[u];
+        acc = fma(D[64 * u], x.x, acc);
+        acc = fma(D[64 * u + 32], x.y, acc);
+      }
+    }
+    return acc;
+  };
+  int par = 0;
+  auto publish = [&](int s, double part) {
+    red[par][q][rl] = part;
+    __syncthreads();
+    const int k0 = bidx(s) * NB;
+    if (t < min(NB, n - k0)) {
+      const double x = (red[par][0][t] + red[par][1][t]) + (red[par][2][t] + red[par][3][t]);
+      if (UPPER || s != withhold)  // a withheld step (failure injection) is never published
+        publish_word(slots + (size_t)s * 256 + 2 * t, tag, x);
+      b[k0 + t] = x;
+    }
+    par ^= 1;
+    if (s + G < nblk) stage(s + G);  // every thread is past Di and m
+  };
+
+  if (g == 0) publish(0, inv_product(0));
+  int used = 0;
+#pragma unroll 1
+  for (int s = 0; s + 1 < nblk; ++s) {
+    const int s2 = first(s);
+    if (s2 >= nblk) break;  // no rows left to update
+    const int cb = min(NB, n - bidx(s) * NB);
+    double z = 0.0;
+    if (s2 == s + 1) {
+      cp_async_all();   // the inverse is there
+      __syncthreads();  // the last step's sums are in wacc
+      z = inv_product(s2);
+    }
+    if (t < NB) ys[t] = t < cb ? poll_word(slots + (size_t)s * 256 + 2 * t, tag, status, wait_ns, &s_abort) : 0.0;
+    __syncthreads();
+    if (s_abort) break;
+    int sx = s2;
+    if (s2 == s + 1) {
+      double a = 0.0;
+#pragma unroll
+      for (int u = 0; u < 32; u += 2) {
+        const double2 y = *reinterpret_cast<const double2*>(ys + 32 * q + u);
+        a = fma(m[u], y.x, a);
+        a = fma(m[u + 1], y.y, a);
+      }
+      publish(s2, z - a);
+      sx += G;
+    }
+#pragma unroll 1
+    for (; sx < nblk; sx += G) {
+      const int h = used & 1;
+      if (!tile_wait(bar_s + 8 * h, (used >> 1) & 1, wait_ns)) {  // seen at the next step
+        atomicCAS(status, 0, BEM_ERR_TIMEOUT);
+        s_abort = 1;
+      }
+      const float* p = ring + h * NB * NB + 32 * q * NB + rl;
+      double a = 0.0;
+#pragma unroll
+      for (int u = 0; u < 32; u += 2) {
+        const double2 y = *reinterpret_cast<const double2*>(ys + 32 * q + u);
+        a = fma((double)p[u * NB], y.x, a);
+        a = fma((double)p[(u + 1) * NB], y.y, a);
+      }
+      red[par][q][rl] = a;
+      __syncthreads();
+      ++used;
+      if (t == 0) fill();  // the tile just read makes room
+      if (t < NB)
+        wacc[((sx - g) / G) * NB + t] -= (red[par][0][t] + red[par][1][t]) + (red[par][2][t] + red[par][3][t]);
+      par ^= 1;
+    }
+  }
+  cp_async_all();
+  if (t == 0)  // copies under way when the sweep was given up
+    for (; used < asked; ++used) tile_wait(bar_s + 8 * (used & 1), (used >> 1) & 1, wait_ns);
 }
 
 // ---- the transposed solve: S^T x = b with the same factors --------------------------
@@ -2222,14 +2504,18 @@ int lu_solve_t_fp64(bem_ctx* c, const double* LU, int64_t lda, int n, double* b)
 }
 
 // Inverses of the diagonal blocks of freshly computed factors, kept in the context for
-// the block-inverse sweeps of lu_solve (2 x 128 KB per 128-row block).
+// the block-inverse sweeps of lu_solve (2 x 128 KB per 128-row block, with FP32 factors as much
+// again for the lead blocks).
 template <typename T>
 int lu_prepare_inverses(bem_ctx* c, const T* S, int64_t lda, int n) {
   c->dinv_src = nullptr;
   if (const char* e = getenv("BEM_SWEEP_INV"))  // 0: keep the substitution sweeps
     if (atoi(e) == 0) return BEM_OK;
+  if (sizeof(T) == 4 && ((reinterpret_cast<uintptr_t>(S) | (uintptr_t)(lda * 4)) & 15) != 0)
+    return BEM_OK;  // no tensor map: the substitution sweeps
   const int nblk = (n + kSolveBlock - 1) / kSolveBlock;
-  const size_t need = (size_t)nblk * 2 * kSolveBlock * kSolveBlock;
+  // FP32 factors: the lead blocks behind the inverses
+  const size_t inv = (size_t)nblk * 2 * kSolveBlock * kSolveBlock, need = sizeof(T) == 4 ? 2 * inv : inv;
   if (c->dinv.count < need) {
     c->dinv.release();
     BEM_CUDA(c, c->dinv.alloc(need));
@@ -2242,6 +2528,15 @@ int lu_prepare_inverses(bem_ctx* c, const T* S, int64_t lda, int n) {
   }
   diag_inv_kernel<T><<<dim3(nblk, 2), kTriThreads, smem, c->stream>>>(S, lda, n, c->dinv.p);
   BEM_LAUNCH_CHECK(c);
+  if constexpr (sizeof(T) == 4) {
+    static DeviceOnce lead_attr;
+    if (lead_attr.pending()) {
+      BEM_CUDA(c, cudaFuncSetAttribute(lead_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeadSmem));
+      lead_attr.mark();
+    }
+    lead_kernel<<<dim3(nblk, 2), kLeadThreads, kLeadSmem, c->stream>>>(S, lda, n, c->dinv.p, c->dinv.p + inv);
+    BEM_LAUNCH_CHECK(c);
+  }
   c->dinv_src = S;
   c->dinv_n = n;
   c->dinv_lda = lda;
@@ -2259,18 +2554,22 @@ int sweep_inv_launch(bem_ctx* c, const T* S, int64_t lda, int n, double* b, unsi
   const int nblk = (n + kSolveBlock - 1) / kSolveBlock;
   const int G = std::min(nblk, c->sm_count);
   const int nown = (nblk + G - 1) / G;
-  const size_t dsm = ((size_t)kSolveBlock * kSolveBlock + (size_t)nown * kSolveBlock) * sizeof(double);
+  constexpr bool f32 = sizeof(T) == 4;
+  const size_t dsm = (f32 ? kSweepInvSmem + 2 * kSweepTileBytes + 128 : kSolveBlock * kSolveBlock * sizeof(double)) +
+                     (size_t)nown * kSolveBlock * sizeof(double);
+  const void* fn;
+  if constexpr (f32) fn = reinterpret_cast<const void*>(&sweep_ring_kernel<UPPER>);
+  else fn = reinterpret_cast<const void*>(&sweep_inv_kernel<UPPER>);
   std::atomic<int>& lim = max_dyn[current_device()];
   if (lim.load() == 0) {
     cudaFuncAttributes fa{};
     int optin = 0;
-    BEM_CUDA(c, cudaFuncGetAttributes(&fa, sweep_inv_kernel<T, UPPER>));
+    BEM_CUDA(c, cudaFuncGetAttributes(&fa, fn));
     BEM_CUDA(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     const int mx = optin - (int)fa.sharedSizeBytes;
-    BEM_CUDA(c, cudaFuncSetAttribute(sweep_inv_kernel<T, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+    BEM_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     int per_sm = 0;
-    BEM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_inv_kernel<T, UPPER>, kSweepThreads,
-                                                              (size_t)mx));
+    BEM_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kSweepThreads, (size_t)mx));
     if (per_sm < 1) return bem_fail(c, BEM_ERR_CUDA, "block-inverse sweep kernel does not fit on an SM");
     lim.store(mx);
   }
@@ -2278,10 +2577,18 @@ int sweep_inv_launch(bem_ctx* c, const T* S, int64_t lda, int n, double* b, unsi
   const double* dinv = c->dinv.p;
   unsigned long long wns = c->wait_ns;
   int withhold = c->withhold_block;
-  void* args[] = {(void*)&S,     (void*)&lda,    (void*)&n,   (void*)&dinv, (void*)&b,
-                  (void*)&slots, (void*)&tag,    (void*)&status, (void*)&wns, (void*)&withhold};
-  BEM_CUDA(c, cudaLaunchCooperativeKernel((void*)sweep_inv_kernel<T, UPPER>, dim3(G), dim3(kSweepThreads), args,
-                                          dsm, c->stream));
+  const double* lead = dinv + (size_t)nblk * 2 * kSolveBlock * kSolveBlock;
+  void* args[10];
+  int k = 0;
+  CUtensorMap map;
+  if constexpr (f32) {
+    if (int rc = tma_map_f32(c, &map, S, n, n, lda, kSolveBlock, kSolveBlock)) return rc;
+    for (void* v : {(void*)&map, (void*)&n, (void*)&dinv, (void*)&lead}) args[k++] = v;
+  } else {
+    for (void* v : {(void*)&S, (void*)&lda, (void*)&n, (void*)&dinv}) args[k++] = v;
+  }
+  for (void* v : {(void*)&b, (void*)&slots, (void*)&tag, (void*)&status, (void*)&wns, (void*)&withhold}) args[k++] = v;
+  BEM_CUDA(c, cudaLaunchCooperativeKernel(fn, dim3(G), dim3(kSweepThreads), args, dsm, c->stream));
   ++c->launches;
   return BEM_OK;
 }

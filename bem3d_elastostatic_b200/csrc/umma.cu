@@ -799,6 +799,17 @@ __global__ void split_b_kernel(int n, int K, const float* __restrict__ B, int64_
 
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
+int load_encode(bem_ctx* c) {
+  if (!g_encode) {
+    cudaDriverEntryPointQueryResult q;
+    void* fn = nullptr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
+      return bem_fail(c, BEM_ERR_CUDA, "cuTensorMapEncodeTiled not available");
+    g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  }
+  return BEM_OK;
+}
+
 bool make_map(CUtensorMap* map, const void* ptr, int rows, int K, int box_rows) {
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)K * 2};
@@ -865,6 +876,20 @@ int umma_setup(bem_ctx* c) {
 
 }  // namespace
 
+int tma_map_f32(bem_ctx* c, CUtensorMap* map, const float* A, int rows, int cols, int64_t ld, int box_rows,
+                int box_cols) {
+  if (int rc = load_encode(c)) return rc;
+  cuuint64_t dims[2] = {(cuuint64_t)rows, (cuuint64_t)cols};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {(cuuint32_t)box_rows, (cuuint32_t)box_cols};
+  cuuint32_t estr[2] = {1, 1};
+  if (g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(A), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return bem_fail(c, BEM_ERR_CUDA, "tensor map encoding of an FP32 matrix failed");
+  return BEM_OK;
+}
+
 bool umma_supported(int K) { return K > 0 && K <= kMaxK && K % UK == 0; }
 
 // Grows the BF16 operand buffer to what an M x N x K update needs (before a captured
@@ -891,13 +916,7 @@ int gemm_umma_bf16(bem_ctx* c, int M, int N, int K, const float* A, int64_t lda,
   if (nprod != 1 && nprod != 3) return bem_fail(c, BEM_ERR_ARG, "umma: nprod must be 1 or 3");
   if (store && nprod != 3) return bem_fail(c, BEM_ERR_ARG, "umma: the storing form takes three products");
   if (!umma_supported(K)) return bem_fail(c, BEM_ERR_ARG, "umma: K must be a multiple of 64 up to 1024");
-  if (!g_encode) {
-    cudaDriverEntryPointQueryResult q;
-    void* fn = nullptr;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn)
-      return bem_fail(c, BEM_ERR_CUDA, "cuTensorMapEncodeTiled not available");
-    g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-  }
+  if (int rc = load_encode(c)) return rc;
   if (int rc = umma_setup(c)) return rc;
   const size_t na = (size_t)M * K, nb_ = (size_t)N * K;
   const size_t need = 2 * (na + nb_) * sizeof(__nv_bfloat16) + 256;

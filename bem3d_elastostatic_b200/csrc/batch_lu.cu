@@ -19,7 +19,7 @@
 //     subtracts the tile times the block solved by the step before, and block k's CTA
 //     multiplies by its inverse (batch_step_kernel).
 //   Residual: one CTA per 128 rows, the columns streamed once for all load cases.
-// Measured on 96 boxes of 78 to 2,598 unknowns with eight load cases: FP32 LU 155 -> 16.5 ms, ten
+// Measured on 96 boxes of 78 to 2,598 unknowns with eight load cases: FP32 LU 155 -> 14.2 ms, ten
 // sweeps 42 -> 6.8 ms, residuals 15.9 -> 2.7 ms.
 #include <algorithm>
 #include <climits>
@@ -169,28 +169,46 @@ __global__ void __launch_bounds__(128) batch_swap_kernel(const SysDev* __restric
   }
 }
 
-// A(t0.., t0..cend) -= A(t0.., j0..j0+k) A(j0..j0+k, t0..cend), k a multiple of 32: tiles of
-// 16 M x 16 M entries, M x M per thread in 16-byte vectors of rows and columns; the tile is
-// loaded with the first operand tiles, so that it costs one memory round trip.  FP32: two CTAs
-// per SM at 128 registers (one at 181 left the loads exposed: 18.9 ms for the 81 launches of the
-// batch above, 13.6 ms with two, 10.8 ms with two panels a step).
+// A(t0.., t0..cend) -= A(t0.., j0..j0+k) A(j0..j0+k, t0..cend), k 32 or 64: tiles of
+// 16 M x 16 M entries, M x M per thread in 16-byte vectors of rows.  Bound by the loads of a tile
+// that no arithmetic covers, so all of them are under way at once: the tile itself to registers,
+// the operand tiles of both 32-step halves to shared memory (cp.async; U12 as it lies, its steps
+// along the fast index).  FP32: two CTAs per SM at 128 registers.  The 81 launches of the batch
+// above: 18.9 ms with one CTA per SM and loads through registers, 13.6 ms with two, 10.8 ms with
+// two panels a step, 8.4 ms with every load ahead (the inner loop rolled: unrolled twice it spills,
+// 9.2 ms).
 template <typename T>
 struct UpdateTile {
   static constexpr int V = 16 / sizeof(T);           // entries per vector
   static constexpr int M = sizeof(T) == 4 ? 8 : 4;   // entries per thread and direction
   static constexpr int TILE = 16 * M;
+  static constexpr int KU = 8 / sizeof(T);           // steps per load of U12
+  static constexpr int PB = kLuNB + V;               // a column's pitch in s_b
+  struct Half {                                      // operands of 32 steps
+    T a[kLuNB][TILE];  // [step][row]
+    T b[TILE][PB];     // [column][step]
+  };
 };
+// 16 bytes global -> shared, zeros unless `in`
+__device__ __forceinline__ void copy_16(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "r"(in ? 16 : 0)
+               : "memory");
+}
 template <typename T>
 __global__ void __launch_bounds__(256, 2) batch_update_kernel(const SysDev* __restrict__ sys,
-                                                           const int* __restrict__ order, T* F, int j0, int k,
+                                                              const int* __restrict__ order, T* F, int j0, int k,
                                                               int t0, int cend) {
   using U = UpdateTile<T>;
-  constexpr int V = U::V, M = U::M, TILE = U::TILE, H = M / V;
+  constexpr int V = U::V, M = U::M, TILE = U::TILE, H = M / V, KU = U::KU;
   struct alignas(16) Vec {
     T v[V];
   };
-  __shared__ __align__(16) T s_a[kLuNB][TILE];
-  __shared__ __align__(16) T s_b[kLuNB][TILE + V];
+  struct alignas(8) Steps {
+    T v[KU];
+  };
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  typename U::Half* sm = reinterpret_cast<typename U::Half*>(smem_raw);  // [k / 32]
   const int s = order[blockIdx.y];
   const int N = sys[s].N, tiles = (N - t0 + TILE - 1) / TILE, C = min(N, cend);
   if ((int)blockIdx.x >= tiles * ((C - t0 + TILE - 1) / TILE)) return;
@@ -199,10 +217,30 @@ __global__ void __launch_bounds__(256, 2) batch_update_kernel(const SysDev* __re
   const int rb = t0 + (blockIdx.x % tiles) * TILE, cb = t0 + (blockIdx.x / tiles) * TILE;
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   // rows up to lda (a multiple of 32, zero beyond N) and columns up to C
+  const int halves = k / kLuNB;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (h < halves) {
+      const int k0 = j0 + h * kLuNB;
+#pragma unroll
+      for (int u = 0; u < kLuNB * TILE / V / 256; ++u) {
+        const int i = tid + u * 256, q = i / (TILE / V), r = (i % (TILE / V)) * V;
+        const bool in = rb + r < lda;
+        copy_16(&sm[h].a[q][r], in ? A + rb + r + (int64_t)(k0 + q) * lda : A, in);
+      }
+#pragma unroll
+      for (int u = 0; u < kLuNB * TILE / V / 256; ++u) {
+        const int i = tid + u * 256, c = i / (kLuNB / V), q = (i % (kLuNB / V)) * V;
+        const bool in = cb + c < C;
+        copy_16(&sm[h].b[c][q], in ? A + k0 + q + (int64_t)(cb + c) * lda : A, in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   T acc[M][M];  // [column][row]
 #pragma unroll
   for (int j = 0; j < M; ++j) {
-    const int c = cb + (j / V) * 16 * V + ty * V + j % V;
+    const int c = cb + ty + 16 * j;
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const int r = rb + h * 16 * V + tx * V;
@@ -212,44 +250,35 @@ __global__ void __launch_bounds__(256, 2) batch_update_kernel(const SysDev* __re
       for (int u = 0; u < V; ++u) acc[j][h * V + u] = x.v[u];
     }
   }
-  for (int k0 = j0; k0 < j0 + k; k0 += kLuNB) {
-    if (k0 > j0) __syncthreads();
-    for (int i = tid; i < kLuNB * TILE / V; i += 256) {
-      const int k = i / (TILE / V), r = (i % (TILE / V)) * V;
-      Vec x{};
-      if (rb + r < lda) x = *reinterpret_cast<const Vec*>(A + rb + r + (int64_t)(k0 + k) * lda);
-      *reinterpret_cast<Vec*>(&s_a[k][r]) = x;
-    }
-    for (int i = tid; i < kLuNB * TILE / V; i += 256) {
-      const int c = i / (kLuNB / V), k = (i % (kLuNB / V)) * V;
-      Vec x{};
-      if (cb + c < C) x = *reinterpret_cast<const Vec*>(A + k0 + k + (int64_t)(cb + c) * lda);
-#pragma unroll
-      for (int u = 0; u < V; ++u) s_b[k + u][c] = x.v[u];
-    }
+  for (int h = 0; h < halves; ++h) {
+    if (h == 0) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-#pragma unroll 2
-    for (int k = 0; k < kLuNB; ++k) {
-      T a[M], b[M];
+    const typename U::Half& S = sm[h];
+#pragma unroll 1
+    for (int q = 0; q < kLuNB; q += KU) {
+      Steps b[M];
 #pragma unroll
-      for (int h = 0; h < H; ++h) {
-        const Vec va = *reinterpret_cast<const Vec*>(&s_a[k][h * 16 * V + tx * V]);
-        const Vec vb = *reinterpret_cast<const Vec*>(&s_b[k][h * 16 * V + ty * V]);
+      for (int j = 0; j < M; ++j) b[j] = *reinterpret_cast<const Steps*>(&S.b[ty + 16 * j][q]);
 #pragma unroll
-        for (int u = 0; u < V; ++u) {
-          a[h * V + u] = va.v[u];
-          b[h * V + u] = vb.v[u];
+      for (int w = 0; w < KU; ++w) {
+        T a[M];
+#pragma unroll
+        for (int g = 0; g < H; ++g) {
+          const Vec va = *reinterpret_cast<const Vec*>(&S.a[q + w][g * 16 * V + tx * V]);
+#pragma unroll
+          for (int u = 0; u < V; ++u) a[g * V + u] = va.v[u];
         }
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+#pragma unroll
+          for (int i = 0; i < M; ++i) acc[j][i] = fma(-a[i], b[j].v[w], acc[j][i]);
       }
-#pragma unroll
-      for (int j = 0; j < M; ++j)
-#pragma unroll
-        for (int i = 0; i < M; ++i) acc[j][i] = fma(-a[i], b[j], acc[j][i]);
     }
   }
 #pragma unroll
   for (int j = 0; j < M; ++j) {
-    const int c = cb + (j / V) * 16 * V + ty * V + j % V;
+    const int c = cb + ty + 16 * j;
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const int r = rb + h * 16 * V + tx * V;
@@ -314,7 +343,8 @@ bool update(BatchSolve& b, T* F, int j0, int k, int t0, int cend) {
   if (left == 0) return true;
   constexpr int TILE = UpdateTile<T>::TILE;
   const int rt = (b.N[0] - t0 + TILE - 1) / TILE, ct = (std::min(b.N[0], cend) - t0 + TILE - 1) / TILE;
-  batch_update_kernel<T><<<dim3(rt * ct, left), 256, 0, b.stream>>>(b.sys, b.order, F, j0, k, t0, cend);
+  batch_update_kernel<T><<<dim3(rt * ct, left), 256, (k / kLuNB) * sizeof(typename UpdateTile<T>::Half), b.stream>>>(
+      b.sys, b.order, F, j0, k, t0, cend);
   ++b.launches;
   return cudaGetLastError() == cudaSuccess;
 }
@@ -866,6 +896,8 @@ template <typename T>
 bool attributes(size_t perm_smem) {
   return cudaFuncSetAttribute(batch_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(kTriElems<double> * sizeof(double))) == cudaSuccess &&
+         cudaFuncSetAttribute(batch_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              2 * (int)sizeof(typename UpdateTile<T>::Half)) == cudaSuccess &&
          cudaFuncSetAttribute(batch_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem) ==
              cudaSuccess;
 }

@@ -90,17 +90,20 @@ def _known_values(mesh: Mesh):
     N = mesh.ndof
     uk = np.zeros(N, dtype=bool)
     vp = np.zeros(N)
-    order = [[] for _ in range(mesh.n)]
-    for e in range(mesh.ne):
-        for k in range(int(mesh.nconec[e])):
-            order[mesh.kconec[k, e] - 1].append((e, k))
-    for i in range(mesh.n):
-        for ld in range(3):
-            for e, k in order[i][:8]:
-                if mesh.kode[3 * e + ld] == 0:
-                    uk[3 * i + ld] = True
-                    vp[3 * i + ld] = mesh.bc[3 * k + ld, e]
-                    break
+    kc = np.asarray(mesh.kconec).T  # (ne, 9)
+    e, k = np.nonzero(np.arange(kc.shape[1]) < np.asarray(mesh.nconec)[:, None])  # by element, then position
+    node = kc[e, k] - 1
+    by_node = np.argsort(node, kind="stable")
+    node, e, k = node[by_node], e[by_node], k[by_node]
+    near = np.arange(node.size) - np.searchsorted(node, node) < 8  # a node's first eight incidences
+    node, e, k = node[near], e[near], k[near]
+    kode, bc = np.asarray(mesh.kode), np.asarray(mesh.bc)
+    for ld in range(3):
+        fixed = np.flatnonzero(kode[3 * e + ld] == 0)
+        first = fixed[np.unique(node[fixed], return_index=True)[1]]
+        dof = 3 * node[first] + ld
+        uk[dof] = True
+        vp[dof] = bc[3 * k[first] + ld, e[first]]
     return uk, vp
 
 

@@ -17,6 +17,7 @@
 //   * to nu through c3..c6, and to mu through the prescribed tractions only (an
 //     unknown traction is mu x, and mu G does not depend on mu).
 // 9-node quadrilateral elements.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -26,7 +27,7 @@
 namespace bem {
 namespace {
 
-constexpr int kRec = 18;  // per (element, Gauss point): y, a1, a2, u(y), t(y), prescribed t(y)
+constexpr int kRec = 22;  // per (element, Gauss point): y, a1, a2, u(y), t(y), prescribed t(y), normal, area
 
 __constant__ double c_f[36][9], c_d1[36][9], c_d2[36][9], c_w[36];
 __constant__ double c_gi6[6], c_om6[6];
@@ -121,10 +122,17 @@ __global__ void adj_table_kernel(int ne, const int* __restrict__ kconec, const i
       if (kode[3 * e + d] != 0) o[15 + d] += c_f[q][k] * tv;
     }
   }
+  const double cr[3] = {o[4] * o[8] - o[5] * o[7], o[5] * o[6] - o[3] * o[8], o[3] * o[7] - o[4] * o[6]};
+  o[21] = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
+  for (int d = 0; d < 3; ++d) o[18 + d] = cr[d] / o[21];
   for (int c = 0; c < kRec; ++c) tab[(int64_t)gid * kRec + c] = o[c];
 }
 
-// regular pairs: CTA = 32 collocation nodes (lanes) x 8 warps over the elements
+// regular pairs: CTA = 32 collocation nodes (lanes) x 8 warps over the elements, of which
+// blockIdx.y takes every gridDim.y-th group of eight.  Bound by the FP64 pipe, so the groups are
+// dealt out until every SM has several CTAs (one CTA per 32 nodes left a third of the SMs idle at
+// 3,076 nodes), and what depends on the element's point alone (area element and normal: a square
+// root and three divisions) comes from the table: 3,076 nodes and 768 elements 5.5 -> 2.6 ms.
 __global__ void __launch_bounds__(256) adj_regular_kernel(int n, int ne, const int* __restrict__ kconec,
                                                           const double* __restrict__ x,
                                                           const double* __restrict__ y,
@@ -141,7 +149,7 @@ __global__ void __launch_bounds__(256) adj_regular_kernel(int n, int ne, const i
   const double ui[3] = {U[3 * ii], U[3 * ii + 1], U[3 * ii + 2]};
   const double li[3] = {active ? lam[3 * ii] : 0.0, active ? lam[3 * ii + 1] : 0.0, active ? lam[3 * ii + 2] : 0.0};
   double gx[3] = {0.0, 0.0, 0.0}, snu = 0.0, smu = 0.0;
-  for (int e = w; e < ne; e += 8) {
+  for (int e = w + 8 * blockIdx.y; e < ne; e += 8 * gridDim.y) {
     int kc[9];
     bool sing = false;
     for (int k = 0; k < 9; ++k) {
@@ -158,10 +166,7 @@ __global__ void __launch_bounds__(256) adj_regular_kernel(int n, int ne, const i
         const double* o = T + q * kRec;
         const double a1[3] = {__ldg(o + 3), __ldg(o + 4), __ldg(o + 5)};
         const double a2[3] = {__ldg(o + 6), __ldg(o + 7), __ldg(o + 8)};
-        const double cr[3] = {a1[1] * a2[2] - a1[2] * a2[1], a1[2] * a2[0] - a1[0] * a2[2],
-                              a1[0] * a2[1] - a1[1] * a2[0]};
-        const double J = sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-        const double nn[3] = {cr[0] / J, cr[1] / J, cr[2] / J};
+        const double J = __ldg(o + 21), nn[3] = {__ldg(o + 18), __ldg(o + 19), __ldg(o + 20)};
         const double rv[3] = {__ldg(o + 0) - xi[0], __ldg(o + 1) - xi[1], __ldg(o + 2) - xi[2]};
         const double du[3] = {__ldg(o + 9) - ui[0], __ldg(o + 10) - ui[1], __ldg(o + 11) - ui[2]};
         const double tq[3] = {__ldg(o + 12), __ldg(o + 13), __ldg(o + 14)};
@@ -358,8 +363,9 @@ int launch_adjoint_gradient(bem_ctx* c, double* lam, double* grad, double* gmat)
   if (rc) return bem_fail(c, rc, "uploading the adjoint tables");
   const Material& M = c->mat;
   const Kelvin K{M.c3, M.c4, M.c5, M.c6, M.mu, M.nu};
-  DBuf<double> tab;
-  BEM_CUDA(c, tab.alloc((size_t)c->ne * 36 * kRec));
+  Kept<unsigned char> ws(c->ip_ws);
+  BEM_CUDA(c, ws.reserve((size_t)c->ne * 36 * kRec * sizeof(double)));
+  double* tab = reinterpret_cast<double*>(c->ip_ws.p);
   if (c->npins > 0) {
     zero_pins_kernel<<<(c->npins + 127) / 128, 128, 0, c->stream>>>(c->pins.p, c->npins, lam);
     BEM_LAUNCH_CHECK(c);
@@ -368,10 +374,12 @@ int launch_adjoint_gradient(bem_ctx* c, double* lam, double* grad, double* gmat)
   BEM_CUDA(c, cudaMemsetAsync(gmat, 0, 2 * sizeof(double), c->stream));
   const int64_t nt = 36 * (int64_t)c->ne;
   adj_table_kernel<<<(unsigned)((nt + 127) / 128), 128, 0, c->stream>>>(c->ne, c->kconec.p, c->kode.p, c->x.p,
-                                                                         c->y.p, c->z.p, c->U.p, c->DFI.p, tab.p);
+                                                                         c->y.p, c->z.p, c->U.p, c->DFI.p, tab);
   BEM_LAUNCH_CHECK(c);
-  adj_regular_kernel<<<(c->n + 31) / 32, 256, 0, c->stream>>>(c->n, c->ne, c->kconec.p, c->x.p, c->y.p, c->z.p,
-                                                               c->U.p, lam, tab.p, K, grad, gmat);
+  const int nodes = (c->n + 31) / 32, groups = (c->ne + 7) / 8;
+  const int split = std::min(groups, (8 * c->sm_count + nodes - 1) / nodes);
+  adj_regular_kernel<<<dim3(nodes, split), 256, 0, c->stream>>>(c->n, c->ne, c->kconec.p, c->x.p, c->y.p, c->z.p,
+                                                               c->U.p, lam, tab, K, grad, gmat);
   BEM_LAUNCH_CHECK(c);
   adj_singular_kernel<<<(8 * c->n + 3) / 4, 128, 0, c->stream>>>(c->n, c->nesim.p, c->ke.p, c->kconec.p, c->kode.p,
                                                                   c->x.p, c->y.p, c->z.p, c->U.p, c->DFI.p, lam, K,

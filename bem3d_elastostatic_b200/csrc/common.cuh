@@ -86,6 +86,20 @@ struct DBuf {
   size_t bytes() const { return count * sizeof(T); }
 };
 
+// A call's use of a workspace that its context keeps: grown when too small, released at the end
+// of the call when it has become larger than kWsKeep.
+template <typename T>
+struct Kept {
+  DBuf<T>& b;
+  explicit Kept(DBuf<T>& buf) : b(buf) {}
+  Kept(const Kept&) = delete;
+  Kept& operator=(const Kept&) = delete;
+  ~Kept() {
+    if (b.bytes() > kWsKeep) b.release();
+  }
+  cudaError_t reserve(size_t n) { return b.count >= n ? cudaSuccess : b.alloc(n); }
+};
+
 // 1 / sqrt(x) from the hardware's approximation of its leading bits and one third-order
 // step: with y (1 + d) = 1 / sqrt(x) and e = 1 - x y^2, y (1 + e/2 + 3/8 e^2) is off by
 // 5/16 e^3, below rounding for the approximation's |e| < 2^-18.  Five FP64 operations; no
@@ -238,7 +252,7 @@ struct bem_ctx {
   // internal points: the tables, partial sums and pair lists of a call, and the pairs'
   // sums; kept up to kWsKeep bytes each for the next call
   bem::DBuf<unsigned char> ip_ws, ip_pairs;
-  bem::DBuf<double> ip_io;  // the host interface's device copies, kept likewise
+  bem::DBuf<double> io;  // the host interfaces' device copies, kept likewise
   bem::DBuf<unsigned char> umma_buf;
   bem::DBuf<int> umma_err;
   // profiling (bem_profile_begin/end)

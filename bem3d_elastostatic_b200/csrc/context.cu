@@ -418,28 +418,30 @@ int bem_dgesv(bem_ctx* c, int n, int nrhs, double* A, int lda, int* ipiv, double
   BEM_CUDA(c, cudaSetDevice(c->device));
   *info = 0;
   const int64_t ld = ((int64_t)n + 31) / 32 * 32;
-  bem::DBuf<double> dA, dB;
-  bem::DBuf<int> dp;
-  if (dA.alloc((size_t)(ld * n)) != cudaSuccess) return bem_fail(c, BEM_ERR_OOM, "dgesv: allocating A");
-  BEM_CUDA(c, dB.alloc((size_t)ld * std::max(nrhs, 1)));
-  BEM_CUDA(c, dp.alloc(n));
-  BEM_CUDA(c, cudaMemcpy2DAsync(dA.p, ld * sizeof(double), A, (size_t)lda * sizeof(double), n * sizeof(double), n,
+  // A, B and the pivots in one buffer of the context's: with the same addresses from call to call
+  // the captured factorisation is replayed (captured anew 3 to 6 ms at 1,500 unknowns)
+  bem::Kept<double> io(c->io);
+  const size_t na = (size_t)ld * n, nb = (size_t)ld * std::max(nrhs, 1);
+  if (io.reserve(na + nb + (size_t)ld / 2) != cudaSuccess) return bem_fail(c, BEM_ERR_OOM, "dgesv: allocating A");
+  double *dA = c->io.p, *dB = dA + na;
+  int* dp = reinterpret_cast<int*>(dB + nb);
+  BEM_CUDA(c, cudaMemcpy2DAsync(dA, ld * sizeof(double), A, (size_t)lda * sizeof(double), n * sizeof(double), n,
                                 cudaMemcpyHostToDevice, c->stream));
   if (nrhs > 0)
-    BEM_CUDA(c, cudaMemcpy2DAsync(dB.p, ld * sizeof(double), B, (size_t)ldb * sizeof(double), n * sizeof(double),
+    BEM_CUDA(c, cudaMemcpy2DAsync(dB, ld * sizeof(double), B, (size_t)ldb * sizeof(double), n * sizeof(double),
                                   nrhs, cudaMemcpyHostToDevice, c->stream));
   double secs = 0.0;
-  int rc = bem::lu_factor_fp64(c, dA.p, ld, n, dp.p, info, &secs);
+  int rc = bem::lu_factor_fp64(c, dA, ld, n, dp, info, &secs);
   if (rc) return rc;
   if (*info == 0)
     for (int j = 0; j < nrhs; ++j)
-      if ((rc = bem::lu_solve_fp64(c, dA.p, ld, n, dB.p + (int64_t)j * ld))) return rc;
+      if ((rc = bem::lu_solve_fp64(c, dA, ld, n, dB + (int64_t)j * ld))) return rc;
   std::vector<int> hp(n);
-  BEM_CUDA(c, cudaMemcpyAsync(hp.data(), dp.p, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  BEM_CUDA(c, cudaMemcpy2DAsync(A, (size_t)lda * sizeof(double), dA.p, ld * sizeof(double), n * sizeof(double), n,
+  BEM_CUDA(c, cudaMemcpyAsync(hp.data(), dp, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  BEM_CUDA(c, cudaMemcpy2DAsync(A, (size_t)lda * sizeof(double), dA, ld * sizeof(double), n * sizeof(double), n,
                                 cudaMemcpyDeviceToHost, c->stream));
   if (nrhs > 0 && *info == 0)
-    BEM_CUDA(c, cudaMemcpy2DAsync(B, (size_t)ldb * sizeof(double), dB.p, ld * sizeof(double), n * sizeof(double),
+    BEM_CUDA(c, cudaMemcpy2DAsync(B, (size_t)ldb * sizeof(double), dB, ld * sizeof(double), n * sizeof(double),
                                   nrhs, cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaStreamSynchronize(c->stream));
   for (int i = 0; i < n; ++i) ipiv[i] = hp[i] + 1;
@@ -473,9 +475,9 @@ int bem_boundary_stresses(bem_ctx* c, double* sigma_elem, double* sigma_node, do
   int rc = bem::launch_reorganize(c);
   if (rc) return rc;
   const size_t ne = c->ne, n = c->n;
-  bem::DBuf<double> d;
-  BEM_CUDA(c, d.alloc(54 * ne + 10 * n));
-  double *se = d.p, *sn = se + 54 * ne, *pr = sn + 6 * n, *v = pr + 3 * n;
+  bem::Kept<double> io(c->io);
+  BEM_CUDA(c, io.reserve(54 * ne + 10 * n));
+  double *se = c->io.p, *sn = se + 54 * ne, *pr = sn + 6 * n, *v = pr + 3 * n;
   if ((rc = bem::launch_boundary_stresses(c, se, sn, pr, v))) return rc;
   if (sigma_elem)
     BEM_CUDA(c, cudaMemcpyAsync(sigma_elem, se, 54 * ne * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -492,12 +494,13 @@ int bem_solve_transposed(bem_ctx* c, double* g) {
     return bem_fail(c, BEM_ERR_STATE, "solve_transposed needs a solve with BEM_PREC_FP64 first");
   BEM_CUDA(c, cudaSetDevice(c->device));
   const size_t N = (size_t)c->nsys;
-  bem::DBuf<double> d;
-  BEM_CUDA(c, d.alloc(N));
-  BEM_CUDA(c, cudaMemcpyAsync(d.p, g, N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  int rc = bem::lu_solve_t_fp64(c, c->A.p, c->lda, (int)N, d.p);
+  bem::Kept<double> io(c->io);
+  BEM_CUDA(c, io.reserve(N));
+  double* d = c->io.p;
+  BEM_CUDA(c, cudaMemcpyAsync(d, g, N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  int rc = bem::lu_solve_t_fp64(c, c->A.p, c->lda, (int)N, d);
   if (rc) return rc;
-  BEM_CUDA(c, cudaMemcpyAsync(g, d.p, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  BEM_CUDA(c, cudaMemcpyAsync(g, d, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaStreamSynchronize(c->stream));
   return BEM_OK;
 }
@@ -510,12 +513,13 @@ int bem_adjoint_gradient(bem_ctx* c, const double* lambda, double* grad_xyz, dou
   int rc = bem::launch_reorganize(c);  // u and t of the current solution
   if (rc) return rc;
   const size_t N = 3 * (size_t)c->n;
-  bem::DBuf<double> d;
-  BEM_CUDA(c, d.alloc(2 * N + 2));
-  BEM_CUDA(c, cudaMemcpyAsync(d.p, lambda, N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  if ((rc = bem::launch_adjoint_gradient(c, d.p, d.p + N, d.p + 2 * N))) return rc;
-  BEM_CUDA(c, cudaMemcpyAsync(grad_xyz, d.p + N, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  BEM_CUDA(c, cudaMemcpyAsync(grad_mat, d.p + 2 * N, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  bem::Kept<double> io(c->io);
+  BEM_CUDA(c, io.reserve(2 * N + 2));
+  double* d = c->io.p;
+  BEM_CUDA(c, cudaMemcpyAsync(d, lambda, N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  if ((rc = bem::launch_adjoint_gradient(c, d, d + N, d + 2 * N))) return rc;
+  BEM_CUDA(c, cudaMemcpyAsync(grad_xyz, d + N, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  BEM_CUDA(c, cudaMemcpyAsync(grad_mat, d + 2 * N, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaStreamSynchronize(c->stream));
   return BEM_OK;
 }
@@ -535,24 +539,21 @@ int bem_internal_points(bem_ctx* c, int l, const double* cx, const double* cy, c
   if (l == 0) return BEM_OK;
   if (!cx || !cy || !cz || !u || !s || !pr || !vm) return bem_fail(c, BEM_ERR_ARG, "internal_points: null");
   BEM_CUDA(c, cudaSetDevice(c->device));
-  if (c->ip_io.count < 16 * (size_t)l) BEM_CUDA(c, c->ip_io.alloc(16 * (size_t)l));
-  double* p = c->ip_io.p;
+  bem::Kept<double> io(c->io);
+  BEM_CUDA(c, io.reserve(16 * (size_t)l));
+  double* p = c->io.p;
   double *dx = p, *dy = p + l, *dz = p + 2 * (size_t)l, *du = p + 3 * (size_t)l, *ds = p + 6 * (size_t)l,
          *dp = p + 12 * (size_t)l, *dv = p + 15 * (size_t)l;
   BEM_CUDA(c, cudaMemcpyAsync(dx, cx, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(dy, cy, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(dz, cz, l * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   int rc = bem::launch_internal_points(c, l, dx, dy, dz, du, ds, dp, dv, flags);
-  if (rc) {
-    if (c->ip_io.bytes() > bem::kWsKeep) c->ip_io.release();
-    return rc;
-  }
+  if (rc) return rc;
   BEM_CUDA(c, cudaMemcpyAsync(u, du, 3 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(s, ds, 6 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(pr, dp, 3 * (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaMemcpyAsync(vm, dv, (size_t)l * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   BEM_CUDA(c, cudaStreamSynchronize(c->stream));
-  if (c->ip_io.bytes() > bem::kWsKeep) c->ip_io.release();
   return BEM_OK;
 }
 

@@ -67,7 +67,7 @@ __global__ void row_scale_kernel(int n, const unsigned long long* __restrict__ r
 // a cycle an SM reads from L2, so the row scales, powers of two, stay in shared memory as
 // their exponents (SMEM; orders whose exponents do not fit read them with the column, which
 // doubles those bytes), and eight 16-byte loads a thread are in flight throughout, the
-// remainder of a column included: 56,448 columns in 7.7 ms, 13.3 ms before.  The FP32
+// remainder of a column included: 56,454 columns in 7.7 ms, 13.3 ms before.  The FP32
 // copy's padding rows are zero.
 constexpr int kColThreads = 1024;
 constexpr int kColLoads = 8;  // double2 per thread and turn

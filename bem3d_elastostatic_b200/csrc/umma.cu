@@ -778,7 +778,7 @@ __device__ __forceinline__ void split_8(const float (&v)[8], __nv_bfloat16* hi, 
 
 // A (m x K, FP32, column-major lda) -> hi/lo BF16 [m][K] (K contiguous); lo nullable.  Transposed
 // through shared memory, 64 rows x 64 K per CTA, so that a row leaves as 128 bytes (a thread per
-// row and eight K wrote 16 bytes every 2 K bytes: 9.9 ms for the 163 splits of a 56,448-unknown
+// row and eight K wrote 16 bytes every 2 K bytes: 9.9 ms for the 163 splits of a 56,454-unknown
 // factorisation, 4.8 ms this way).
 constexpr int kSplit = 64;
 __global__ void __launch_bounds__(256) split_a_kernel(int m, int K, const float* __restrict__ A, int64_t lda,

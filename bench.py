@@ -461,7 +461,7 @@ def leg_batch(device):
         t0 = time.perf_counter()
         b.assemble()
         t_asm = time.perf_counter() - t0
-        b.solve("fp32-ir", tol=1e-15, max_iter=10)  # warm-up: autotune + graph capture
+        b.solve("fp32-ir", tol=1e-15, max_iter=10)  # warm-up: graph capture
         ir = b.solve("fp32-ir", tol=1e-15, max_iter=10)
         x_ir = [b.solution(i) for i in range(len(systems))]
         b.solve("fp64")

@@ -2059,11 +2059,13 @@ __device__ __forceinline__ bool tile_ready(unsigned bar, unsigned parity) {
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool tile_wait(unsigned bar, unsigned parity, unsigned long long wait_ns) {
+// false when the wait runs out, or at once when `status` (nullable) holds an error
+__device__ __forceinline__ bool tile_wait(unsigned bar, unsigned parity, unsigned long long wait_ns,
+                                          const int* status) {
   if (tile_ready(bar, parity)) return true;
   const unsigned long long t0 = globaltimer_ns();
   while (!tile_ready(bar, parity))
-    if (globaltimer_ns() - t0 > wait_ns) return false;
+    if (globaltimer_ns() - t0 > wait_ns || (status && *((volatile const int*)status) != 0)) return false;
   return true;
 }
 
@@ -2227,10 +2229,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 #pragma unroll 1
     for (; sx < nblk; sx += G) {
       const int h = used & 1;
-      if (!tile_wait(bar_s + 8 * h, (used >> 1) & 1, wait_ns)) {  // seen at the next step
-        atomicCAS(status, 0, BEM_ERR_TIMEOUT);
-        s_abort = 1;
-      }
+      // a wait that runs out only records the error: the next poll that has to wait ends the sweep
+      if (!tile_wait(bar_s + 8 * h, (used >> 1) & 1, wait_ns, status)) atomicCAS(status, 0, BEM_ERR_TIMEOUT);
       const float* p = ring + h * NB * NB + 32 * q * NB + rl;
       double a = 0.0;
 #pragma unroll
@@ -2250,7 +2250,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   }
   cp_async_all();
   if (t == 0)  // copies under way when the sweep was given up
-    for (; used < asked; ++used) tile_wait(bar_s + 8 * (used & 1), (used >> 1) & 1, wait_ns);
+    for (int k = max(0, asked - 2); k < asked; ++k) tile_wait(bar_s + 8 * (k & 1), (k >> 1) & 1, wait_ns, nullptr);
 }
 
 // ---- the transposed solve: S^T x = b with the same factors --------------------------

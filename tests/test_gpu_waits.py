@@ -1,0 +1,43 @@
+"""Bounded device waits that run out: the call returns BEM_ERR_TIMEOUT, and the context solves
+correctly afterwards.  The waits are made to run out by a message that its sender withholds.
+
+Bar of the solves that follow: the backward error ||b - A x|| / (||A|| ||x|| + ||b||) at 1e-14
+(FP64 rounding of a residual at these orders)."""
+import numpy as np
+import pytest
+
+from bem3d_elastostatic_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, seed=3):
+    rng = np.random.default_rng(seed)
+    A = rng.standard_normal((n, n), dtype=np.float32).astype(np.float64) / np.sqrt(n)
+    A[np.diag_indices(n)] += 3.0
+    return np.asfortranarray(A), rng.standard_normal(n)
+
+
+def _backward_error(A, x, b):
+    return np.abs(b - A @ x).max() / (np.abs(A).sum(1).max() * np.abs(x).max() + np.abs(b).max())
+
+
+# the first, an inner and the last block that is waited for; one owned block a CTA and two (more
+# than 148 blocks)
+@pytest.mark.parametrize("n,blocks", [(1000, [0, 6]), (4000, [0, 5, 30]), (148 * 128 + 300, [60, 149])])
+def test_withheld_sweep_block(n, blocks):
+    from bem3d_elastostatic_b200.api import solve_system
+
+    A, b = _system(n)
+    ctx = _lib.Context(0)
+    for block in blocks:
+        ctx.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 100)
+        ctx.set_option(_lib.BEM_OPT_WITHHOLD_BLOCK, block)
+        with pytest.raises(_lib.BemError) as exc:
+            solve_system(A, b, "fp32-ir", ctx=ctx)
+        assert exc.value.code == _lib.BEM_ERR_TIMEOUT
+    ctx.set_option(_lib.BEM_OPT_WITHHOLD_BLOCK, -1)
+    ctx.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 2000)
+    x, _ = solve_system(A, b, "fp32-ir", ctx=ctx)
+    assert _backward_error(A, x, b) <= 1e-14
+    ctx.close()

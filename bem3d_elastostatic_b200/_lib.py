@@ -41,6 +41,7 @@ BEM_OPT_WAIT_LIMIT_MS = 2
 BEM_OPT_WITHHOLD_BLOCK = 3
 BEM_OPT_RESIDUAL = 4
 BEM_OPT_PANEL_WIDTH = 5
+BEM_OPT_WITHHOLD_PIVOT = 6
 
 # every symbol the header declares, for the export check
 EXPORTS = [
@@ -206,7 +207,7 @@ class Context:
 
     def set_option(self, option: int, value: int):
         """bem_set_option: BEM_OPT_PIVOTING, BEM_OPT_WAIT_LIMIT_MS, BEM_OPT_WITHHOLD_BLOCK,
-        BEM_OPT_RESIDUAL, BEM_OPT_PANEL_WIDTH."""
+        BEM_OPT_WITHHOLD_PIVOT, BEM_OPT_RESIDUAL, BEM_OPT_PANEL_WIDTH."""
         self.check(self.L.bem_set_option(self.h, int(option), int(value)), "set_option")
 
     def profile_begin(self, timing=True):

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(kPanelNT, 1)
   const int64_t lda = sys[s].lda;
   T* A = F + sys[s].f_off;
   const int base = j0 + rank * Sm::kLines, nl = max(0, min(Sm::kLines, N - base));
-  const PanelStep P{N, j0, w, piv + sys[s].piv_off, info + s, kPanelWait};
+  const PanelStep P{N, j0, w, piv + sys[s].piv_off, info + s, kPanelWait, -1};
   const bool ok = panel_on_cluster<T, LPT, kPanelNT>(P, sm, C, rank, base, nl, [&](T(&v)[LPT][kPanelW]) {
 #pragma unroll
     for (int q = 0; q < LPT; ++q)

@@ -243,9 +243,9 @@ struct bem_ctx {
   bool lu_window = false;
   int pivot_pref = BEM_PIVOT_WINDOW;  // BEM_OPT_PIVOTING
   // bounded device waits (BEM_OPT_WAIT_LIMIT_MS), in ns, and the test-only withheld
-  // sweep block (BEM_OPT_WITHHOLD_BLOCK, -1 = none)
+  // sweep block and pivot step (BEM_OPT_WITHHOLD_BLOCK, _PIVOT, -1 = none)
   unsigned long long wait_ns = 2000000000ull;
-  int withhold_block = -1;
+  int withhold_block = -1, withhold_pivot = -1;
   int panel_width = 0;  // FP32 factorisation panel width of the *_IR modes (0: the mode's own)
   int f32_gemm_override = -1;  // BEM_F32_GEMM environment override (0, 1, 3)
   // tcgen05 trailing update: BF16 hi/lo operand copies and its error word

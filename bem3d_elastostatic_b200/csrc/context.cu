@@ -173,6 +173,10 @@ int bem_set_option(bem_ctx* c, int option, int64_t value) {
       if (value < -1 || value > INT32_MAX) return bem_fail(c, BEM_ERR_ARG, "set_option: bad block index");
       c->withhold_block = (int)value;
       return BEM_OK;
+    case BEM_OPT_WITHHOLD_PIVOT:
+      if (value < -1 || value > INT32_MAX) return bem_fail(c, BEM_ERR_ARG, "set_option: bad pivot index");
+      c->withhold_pivot = (int)value;
+      return BEM_OK;
     default:
       return bem_fail(c, BEM_ERR_ARG, "set_option: unknown option");
   }

@@ -770,12 +770,15 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // Applies swaps k0+t <-> piv[k0+t] (t = 0..w-1 in order) to rows [a0,a1) and [b0,b1).
 // With window pivoting `win` (nullable) holds the factored w x w diagonal block of the
 // sub-panel (leading dimension kPanelW), which CTA 0 copies into S(k0.., k0..) first;
-// the swaps below touch no row of that block.
+// the swaps below touch no row of that block.  n: the order of S, the pivots' bound.
 template <typename T>
-__global__ void swap_rows_kernel(T* S, int64_t lda, const int* piv, int k0, int w, int a0, int a1, int b0,
+__global__ void swap_rows_kernel(T* S, int64_t lda, int n, const int* piv, int k0, int w, int a0, int a1, int b0,
                                  int b1, const T* win) {
   __shared__ int sp[kPanelW];
-  if (threadIdx.x < w) sp[threadIdx.x] = piv[k0 + threadIdx.x];
+  if (threadIdx.x < w) {
+    const int k = k0 + threadIdx.x;
+    sp[threadIdx.x] = checked_index(piv[k], k, n, k);
+  }
   if (win && blockIdx.x == 0)
     for (int i = threadIdx.x; i < w * w; i += blockDim.x) {
       const int j = i % w, cc = i / w;
@@ -825,7 +828,7 @@ __global__ void __launch_bounds__(256) permute_panel_kernel(T* S, int64_t lda, c
     const int hw = min(kPermMax, w - h0), kh = k0 + h0;
     for (int c = tid; c < hw; c += blockDim.x) {
       perm[c] = c;
-      sp[c] = piv[kh + c] - kh;
+      sp[c] = checked_index(piv[kh + c] - kh, c, hw, c);
     }
     if (tid == 0) nmoved = 0;
     __syncthreads();
@@ -1372,7 +1375,7 @@ static int lu_factor_enqueue(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int
       const int64_t rows = (int64_t)(a1 - a0) + (b1 - b0);
       if (rows > 0 || window) {
         swap_rows_kernel<T><<<(unsigned)std::max<int64_t>(1, (rows + 255) / 256), 256, 0, c->stream>>>(
-            S, lda, piv, r0, w, a0, a1, b0, b1, window ? reinterpret_cast<const T*>(ws.cand_col) : nullptr);
+            S, lda, n, piv, r0, w, a0, a1, b0, b1, window ? reinterpret_cast<const T*>(ws.cand_col) : nullptr);
         BEM_LAUNCH_CHECK(c);
       }
       prof.end(c->stream);
@@ -1538,7 +1541,7 @@ int lu_factor(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int nb,
                                   (long long)(uintptr_t)ws.cand_val, (long long)(uintptr_t)c->umma_buf.p,
                                   (long long)c->umma_buf.count, (long long)(uintptr_t)c->umma_err.p,
                                   c->f32_gemm, c->f64_gemm, prof.on, prof.trailing_only, c->sm_count,
-                                  c->lu_window ? 1 : 0};
+                                  c->lu_window ? 1 : 0, c->withhold_pivot};
   };
   int rc = BEM_OK;
   if (c->lu_graph_off) {

@@ -56,6 +56,13 @@ int lu_factor_ws(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int 
 template <typename T>
 int lu_solve_ws(bem_ctx* c, const T* S, int64_t lda, int n, const int* perm, double* b, double* work);
 
+// A pivot or interchange word as its readers take it: after a wait that ran out in the launch that
+// should have written it, it is whatever the buffer held, and the launches up to the host's look at
+// the error word must stay inside the matrix.
+__host__ __device__ constexpr int checked_index(int v, int lo, int hi, int self) {
+  return v >= lo && v < hi ? v : self;
+}
+
 // the FP64 sub-panel on one cluster (panel64.cu)
 int panel_cluster_lines();
 int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status, int* moved);

@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(128) panel_rows_kernel(double* S, int64_t lda,
   const int tid = threadIdx.x, b1 = r0 + w;
   bool any = false;
   if (tid < W) {
-    s_src[tid] = tid < w ? moved[tid] : r0 + tid;
-    s_dst[tid] = tid < w ? moved[W + tid] : r0 + tid;
+    s_src[tid] = tid < w ? checked_index(moved[tid], r0, n, r0 + tid) : r0 + tid;
+    s_dst[tid] = tid < w ? checked_index(moved[W + tid], r0, n, r0 + tid) : r0 + tid;
     any = s_src[tid] != r0 + tid;
   }
   for (int i = tid; i < W * W; i += 128) {
@@ -138,7 +138,7 @@ int panel_cluster_lines() {
 // panel_cluster_lines().  moved (64 ints) receives its interchanges as panel_rows takes them.
 int panel_cluster_launch(bem_ctx* c, double* S, int64_t lda, int n, int r0, int w, int* piv, int* status,
                          int* moved) {
-  const PanelArgs P{{n, r0, w, piv, status + 1, c->wait_ns}, S, lda, status, moved};
+  const PanelArgs P{{n, r0, w, piv, status + 1, c->wait_ns, c->withhold_pivot}, S, lda, status, moved};
   const int lines = n - r0;
   if (lines > kMaxCluster * 512) return launch<2, 384>(c, P, kMaxCluster);
   if (lines > kMaxCluster * 256) return launch<1, 512>(c, P, kMaxCluster);

@@ -14,8 +14,10 @@
 //     CTA d with st.async, which completes on that CTA's mbarrier: one one-way trip per
 //     pivot, no cluster barrier.  Two slots by step parity suffice: a CTA sends step t + 1
 //     only after its threads have read step t - 1's line.
-// Waits are bounded by the caller's limit; on a timeout the CTA records it, ends its steps and
-// meets the others at the final cluster barrier.
+// Waits are bounded by the caller's limit; on a timeout the CTA records it, ends its steps before
+// it sends again and meets the others at the final cluster barrier: no message is younger than the
+// limit then.  The launches that follow run all the same, so the readers of a panel's pivots and
+// interchanges take them through checked_index (lu.cuh).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -154,6 +156,7 @@ struct PanelStep {
   int* piv;
   int* info;
   unsigned long long wait_ns;
+  int withhold;  // failure injection: the step whose line the first CTA does not send (-1: none)
 };
 
 // Steps [t0, t0 + 8) with LEN = 32 - t0 values left per line: the update shrinks with the
@@ -176,6 +179,7 @@ __device__ __forceinline__ bool panel_steps(const PanelStep& P, PanelSmem<T, LPT
   const int t0 = kPanelW - LEN;
   constexpr int kDest = (kMaxCluster + NW - 1) / NW;  // CTAs a warp sends to
   const unsigned own = smem_u32(&sm);
+  const int hold = rank == 0 ? P.withhold : -1;
   unsigned remote[kDest];
 #pragma unroll
   for (int i = 0; i < kDest; ++i) remote[i] = wp + i * NW < C ? mapa(own, wp + i * NW) : 0u;
@@ -231,7 +235,7 @@ __device__ __forceinline__ bool panel_steps(const PanelStep& P, PanelSmem<T, LPT
       const Key best = sm.cand_key[par][wl];
 #pragma unroll
       for (int i = 0; i < kDest; ++i)
-        if (wp + i * NW < C) {
+        if (wp + i * NW < C && k != hold) {
           const unsigned rb = remote[i] + (smem_u32(&sm.bar[par]) - own);
           st_async(remote[i] + (smem_u32(&sm.slot[par][rank][lane]) - own), x, rb);
           if (lane == 0) st_async_key(remote[i] + (smem_u32(&sm.slot_key[par][rank]) - own), best, rb);
@@ -290,7 +294,7 @@ __device__ __forceinline__ bool panel_steps(const PanelStep& P, PanelSmem<T, LPT
     if (tid == 0) {
       if (C > 1 && t + 2 < P.w && mbar_try(smem_u32(&sm.bar[par]), (t >> 1) & 1))
         mbar_expect(smem_u32(&sm.bar[par]), (unsigned)C * kMsgBytes<T>);  // for step t + 2
-      if (rank == 0 && p < P.n) {
+      if (rank == 0 && p >= k && p < P.n) {
         P.piv[k] = p;
         if (pv == T(0) && *P.info == 0) *P.info = k + 1;
       }

@@ -118,6 +118,10 @@ int bem_get_stream(bem_ctx* ctx, void** stream);
  *                           (-1, the default, publishes all), so that the waits for it run
  *                           out and the solve returns BEM_ERR_TIMEOUT with the context
  *                           still usable
+ *   BEM_OPT_WITHHOLD_PIVOT  failure injection for tests, likewise: the cluster that factors
+ *                           a sub-panel of an FP64 factorisation does not send the pivot
+ *                           line of this step (0-based; sub-panels of more than 256 lines,
+ *                           which take more than one CTA)
  *   BEM_OPT_PANEL_WIDTH     panel width of the FP32 factorisations of the *_IR modes: a
  *                           multiple of 128 up to 1024, or 0 (default) for the mode's
  *                           own (1024 for BEM_PREC_BF16_IR, 512 for BEM_PREC_FP32_IR) */
@@ -126,6 +130,7 @@ int bem_get_stream(bem_ctx* ctx, void** stream);
 #define BEM_OPT_WITHHOLD_BLOCK 3
 #define BEM_OPT_RESIDUAL 4
 #define BEM_OPT_PANEL_WIDTH 5
+#define BEM_OPT_WITHHOLD_PIVOT 6
 int bem_set_option(bem_ctx* ctx, int option, int64_t value);
 
 /* Input: replaces input_data (io_mod.f90:36-146) and update_material_constants

@@ -22,6 +22,26 @@ def _backward_error(A, x, b):
     return np.abs(b - A @ x).max() / (np.abs(A).sum(1).max() * np.abs(x).max() + np.abs(b).max())
 
 
+# the first sub-panel, an inner one and the last with two CTAs; of a fresh workspace and a used one
+@pytest.mark.parametrize("n,pivots", [(300, [0]), (1500, [0, 700, 1219]), (9000, [40])])
+def test_withheld_pivot(n, pivots):
+    from bem3d_elastostatic_b200.api import solve_system
+
+    A, b = _system(n)
+    ctx = _lib.Context(0)
+    for pivot in pivots:
+        ctx.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 100)
+        ctx.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, pivot)
+        with pytest.raises(_lib.BemError) as exc:
+            solve_system(A, b, "fp64", ctx=ctx)
+        assert exc.value.code == _lib.BEM_ERR_TIMEOUT
+    ctx.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, -1)
+    ctx.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 2000)
+    x, _ = solve_system(A, b, "fp64", ctx=ctx)
+    assert _backward_error(A, x, b) <= 1e-14
+    ctx.close()
+
+
 # the first, an inner and the last block that is waited for; one owned block a CTA and two (more
 # than 148 blocks)
 @pytest.mark.parametrize("n,blocks", [(1000, [0, 6]), (4000, [0, 5, 30]), (148 * 128 + 300, [60, 149])])

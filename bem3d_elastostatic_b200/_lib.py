@@ -52,6 +52,7 @@ EXPORTS = [
     "bem_reorganize", "bem_boundary_stresses", "bem_solve_transposed", "bem_adjoint_gradient", "bem_internal_points", "bem_device_state",
     "bem_internal_points_device", "bem_profile_begin", "bem_profile_end",
     "bem_dgesv_noalloc", "bem_batch_create", "bem_batch_destroy", "bem_batch_last_error",
+    "bem_batch_set_option",
     "bem_batch_add", "bem_batch_assemble", "bem_batch_solve", "bem_batch_get_solution",
     "bem_batch_get_system", "bem_batch_launches",
 ]
@@ -155,6 +156,7 @@ def load(build_if_needed: bool = True):
     L.bem_batch_destroy.argtypes = [_vp]
     L.bem_batch_last_error.argtypes = [_vp]
     L.bem_batch_last_error.restype = C.c_char_p
+    L.bem_batch_set_option.argtypes = [_vp, C.c_int, C.c_int64]
     L.bem_batch_add.argtypes = [_vp, C.c_int, C.c_int, _vp, _vp, _vp, _vp, _vp, C.c_double, C.c_double,
                                 _vp, C.c_int, _vp, C.c_int, _vp]
     L.bem_batch_assemble.argtypes = [_vp]

@@ -214,6 +214,10 @@ class Batch:
         self.nrhs.append(len(bcs))
         return idx
 
+    def set_option(self, option: int, value: int):
+        """bem_batch_set_option: BEM_OPT_WAIT_LIMIT_MS, BEM_OPT_WITHHOLD_PIVOT."""
+        self._check(self.L.bem_batch_set_option(self.h, int(option), int(value)), "batch_set_option")
+
     def assemble(self):
         self._check(self.L.bem_batch_assemble(self.h), "batch_assemble")
 

@@ -135,6 +135,8 @@ struct bem_batch {
   int graph_key[3] = {-1, -1, -1};
   double graph_tol = -1.0;
   long long graph_launches = 0;
+  unsigned long long wait_ns = 2000000000ull;  // BEM_OPT_WAIT_LIMIT_MS
+  int withhold_pivot = -1;                     // BEM_OPT_WITHHOLD_PIVOT
   int lu_threads = 0;  // CTA size of the LU the solve took
   // the solutions of the latest solve on the host (pinned), fetched with the first one asked for
   double* host_x = nullptr;
@@ -533,6 +535,24 @@ int bem_batch_assemble(bem_batch* b) {
 
 extern "C" {
 
+int bem_batch_set_option(bem_batch* b, int option, int64_t value) {
+  if (!b) return BEM_ERR_ARG;
+  if (option == BEM_OPT_WAIT_LIMIT_MS) {
+    if (value < 1 || value > 60000) return bfail(b, BEM_ERR_ARG, "batch_set_option: wait limit must be 1..60000 ms");
+    b->wait_ns = (unsigned long long)value * 1000000ull;
+  } else if (option == BEM_OPT_WITHHOLD_PIVOT) {
+    if (value < -1 || value > INT32_MAX) return bfail(b, BEM_ERR_ARG, "batch_set_option: bad pivot index");
+    b->withhold_pivot = (int)value;
+  } else {
+    return bfail(b, BEM_ERR_ARG, "batch_set_option: unknown option");
+  }
+  if (b->graph) {  // captured with the former value
+    cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+  }
+  return BEM_OK;
+}
+
 int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_batch_info* info) {
   if (!b || !b->assembled) return bfail(b, BEM_ERR_STATE, "batch_solve before batch_assemble");
   b->host_valid = false;
@@ -583,6 +603,8 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
     S.conv = b->conv.p;
     S.moved = b->moved.p;
     S.err = b->lu_err.p;
+    S.wait_ns = b->wait_ns;
+    S.withhold_pivot = b->withhold_pivot;
     S.nsys = ns;
     const int cap = precision == BEM_PREC_FP64 ? bem::batch_lu_max_order<double>() : bem::batch_lu_max_order<float>();
     b->lu_threads = S.N[0] <= cap ? 256 : 512;

@@ -40,6 +40,8 @@ struct BatchSolve {
   int *info, *conv;    // per system
   int* moved;          // [systems][64]: the interchanges of the current panel
   int* err;            // one error word
+  unsigned long long wait_ns;  // limit of the panels' waits
+  int withhold_pivot;  // BEM_OPT_WITHHOLD_PIVOT
   int nsys;
   long long launches;  // counted by the calls below
 };

@@ -33,14 +33,13 @@ namespace {
 
 constexpr int kLuNB = 32;  // panel width
 constexpr int kPanelNT = 256;
-constexpr unsigned long long kPanelWait = 2000000000ull;
 
 // ---- LU ----------------------------------------------------------------------------------
 
 template <typename T, int LPT>
 __global__ void __launch_bounds__(kPanelNT, 1)
     batch_panel_kernel(const SysDev* __restrict__ sys, const int* __restrict__ order, T* F, int j0, int C, int* piv,
-                       int* info, int* moved, int* err) {
+                       int* info, int* moved, int* err, unsigned long long wait_ns, int withhold) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using Sm = PanelSmem<T, LPT, kPanelNT>;
   Sm& sm = *reinterpret_cast<Sm*>(smem_raw);
@@ -50,7 +49,7 @@ __global__ void __launch_bounds__(kPanelNT, 1)
   const int64_t lda = sys[s].lda;
   T* A = F + sys[s].f_off;
   const int base = j0 + rank * Sm::kLines, nl = max(0, min(Sm::kLines, N - base));
-  const PanelStep P{N, j0, w, piv + sys[s].piv_off, info + s, kPanelWait, -1};
+  const PanelStep P{N, j0, w, piv + sys[s].piv_off, info + s, wait_ns, withhold};
   const bool ok = panel_on_cluster<T, LPT, kPanelNT>(P, sm, C, rank, base, nl, [&](T(&v)[LPT][kPanelW]) {
 #pragma unroll
     for (int q = 0; q < LPT; ++q)
@@ -94,8 +93,8 @@ __global__ void __launch_bounds__(128) batch_swap_kernel(const SysDev* __restric
   T* A = F + sys[s].f_off;
   bool any = false;
   if (tid < kLuNB) {
-    s_src[tid] = tid < w ? moved[64 * s + tid] : j0 + tid;
-    s_dst[tid] = tid < w ? moved[64 * s + 32 + tid] : j0 + tid;
+    s_src[tid] = tid < w ? checked_index(moved[64 * s + tid], j0, N, j0 + tid) : j0 + tid;
+    s_dst[tid] = tid < w ? checked_index(moved[64 * s + 32 + tid], j0, N, j0 + tid) : j0 + tid;
     any = s_src[tid] != j0 + tid;
   }
   for (int i = tid; i < kLuNB * kLuNB; i += 128) {
@@ -298,7 +297,8 @@ template <typename T, int LPT>
 bool panel_step(BatchSolve& b, T* F, int j0, int active, int C) {
   ++b.launches;
   return launch_clusters(batch_panel_kernel<T, LPT>, active, C, kPanelNT, sizeof(PanelSmem<T, LPT, kPanelNT>),
-                         b.stream, b.sys, b.order, F, j0, C, b.piv, b.info, b.moved, b.err) == cudaSuccess;
+                         b.stream, b.sys, b.order, F, j0, C, b.piv, b.info, b.moved, b.err, b.wait_ns,
+                         b.withhold_pivot) == cudaSuccess;
 }
 
 // systems (the first ones in order) of at least n rows
@@ -580,8 +580,8 @@ __global__ void __launch_bounds__(256) batch_perm_kernel(const SysDev* __restric
   __syncthreads();
   if (threadIdx.x == 0)
     for (int j = 0; j < S.N; ++j) {
-      const int p = s_p[j];
-      if (p != j && p < S.N) {
+      const int p = checked_index(s_p[j], j, S.N, j);
+      if (p != j) {
         const int t = s_l[j];
         s_l[j] = s_l[p];
         s_l[p] = t;

@@ -262,6 +262,10 @@ typedef struct {
 int bem_batch_create(bem_batch** batch, int device);
 int bem_batch_destroy(bem_batch* batch);
 const char* bem_batch_last_error(const bem_batch* batch);
+/* BEM_OPT_WAIT_LIMIT_MS (the waits of the panel factorisation, default 2000 ms) and
+ * BEM_OPT_WITHHOLD_PIVOT (in every system; the largest must have more than 256 unknowns),
+ * as bem_set_option's */
+int bem_batch_set_option(bem_batch* batch, int option, int64_t value);
 /* adds one system (arguments as bem_set_mesh / bem_set_material / bem_set_bc /
  * bem_set_pins; bc holds nrhs load cases, nrhs <= 8 and the same for every system);
  * returns the system's index (>= 0) or an error (< 0) */

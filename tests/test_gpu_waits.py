@@ -42,6 +42,30 @@ def test_withheld_pivot(n, pivots):
     ctx.close()
 
 
+# the first panel of a step and the second; one, two and four rows per thread come with the orders
+@pytest.mark.parametrize("precision", ["fp32-ir", "fp64"])
+@pytest.mark.parametrize("ks,pivot", [([3, 1, 4], 0), ([6] * 5 + [2], 45), ([6] * 44, 33)])
+def test_batch_withheld_pivot(ks, pivot, precision):
+    from bem3d_elastostatic_b200.api import Batch
+    from bem3d_elastostatic_b200.mesh import loaded_box
+
+    rng = np.random.default_rng(len(ks))
+    b = Batch()
+    for k in ks:
+        b.add(*loaded_box(*rng.uniform(0.7, 1.5, 3), k, rng.uniform(0.1, 0.4), 1.0, rng.standard_normal((2, 3))))
+    b.assemble()
+    b.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 50)
+    b.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, pivot)
+    for _ in range(2):  # captured and replayed
+        with pytest.raises(_lib.BemError) as exc:
+            b.solve(precision)
+        assert exc.value.code == _lib.BEM_ERR_TIMEOUT
+    b.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, -1)
+    b.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 2000)
+    assert b.solve(precision)["max_backward_error"] <= 1e-14
+    b.close()
+
+
 # the first, an inner and the last block that is waited for; one owned block a CTA and two (more
 # than 148 blocks)
 @pytest.mark.parametrize("n,blocks", [(1000, [0, 6]), (4000, [0, 5, 30]), (148 * 128 + 300, [60, 149])])

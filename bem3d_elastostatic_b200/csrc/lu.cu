@@ -1511,8 +1511,8 @@ int lu_factor_ws(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int 
 }
 
 // The context's factorisation: workspace kept in the context, the launch sequence
-// captured once per (factors, order, panel width, workspace, GEMM buffers, profile mode)
-// and replayed, then the diagonal-block inverses of the solve.  Capture that the
+// captured once per (factors, order, panel width, workspace, GEMM buffers, profile mode, wait
+// limit) and replayed, then the diagonal-block inverses of the solve.  Capture that the
 // runtime refuses (or BEM_LU_GRAPH=0) leaves plain launches.
 template <typename T>
 int lu_factor(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int nb, int* info) {
@@ -1541,7 +1541,7 @@ int lu_factor(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int nb,
                                   (long long)(uintptr_t)ws.cand_val, (long long)(uintptr_t)c->umma_buf.p,
                                   (long long)c->umma_buf.count, (long long)(uintptr_t)c->umma_err.p,
                                   c->f32_gemm, c->f64_gemm, prof.on, prof.trailing_only, c->sm_count,
-                                  c->lu_window ? 1 : 0, c->withhold_pivot};
+                                  c->lu_window ? 1 : 0, c->withhold_pivot, (long long)c->wait_ns};
   };
   int rc = BEM_OK;
   if (c->lu_graph_off) {

@@ -42,6 +42,27 @@ def test_withheld_pivot(n, pivots):
     ctx.close()
 
 
+def test_wait_limit_of_a_replayed_factorisation():
+    """The limit in force is the one set last, also for a factorisation captured before."""
+    import time
+
+    from bem3d_elastostatic_b200.api import solve_system
+
+    A, b = _system(600)
+    ctx = _lib.Context(0)
+    ctx.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, 0)
+    seconds = []
+    for limit in (1500, 50, 1500):
+        ctx.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, limit)
+        t = time.perf_counter()
+        with pytest.raises(_lib.BemError):
+            solve_system(A, b, "fp64", ctx=ctx)
+        seconds.append(time.perf_counter() - t)
+    assert seconds[0] >= 1.5 and seconds[2] >= 1.5  # one wait runs out per solve
+    assert seconds[1] <= 1.0
+    ctx.close()
+
+
 # the first panel of a step and the second; one, two and four rows per thread come with the orders
 @pytest.mark.parametrize("precision", ["fp32-ir", "fp64"])
 @pytest.mark.parametrize("ks,pivot", [([3, 1, 4], 0), ([6] * 5 + [2], 45), ([6] * 44, 33)])

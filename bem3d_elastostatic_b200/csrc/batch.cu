@@ -628,6 +628,7 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
     b->graph_key[1] = sweeps;
     b->graph_tol = tol;
   }
+  b->factored = false;  // until this solve has succeeded: it writes over the last one's vectors
   cudaEvent_t e0, e1;
   BB_CUDA(b, cudaEventCreate(&e0));
   BB_CUDA(b, cudaEventCreate(&e1));

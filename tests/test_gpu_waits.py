@@ -106,3 +106,25 @@ def test_withheld_sweep_block(n, blocks):
     x, _ = solve_system(A, b, "fp32-ir", ctx=ctx)
     assert _backward_error(A, x, b) <= 1e-14
     ctx.close()
+
+
+def test_no_solution_of_a_failed_batch_solve():
+    from bem3d_elastostatic_b200.api import Batch
+    from bem3d_elastostatic_b200.mesh import loaded_box
+
+    b = Batch()
+    b.add(*loaded_box(1.0, 0.8, 1.2, 4, 0.3))
+    b.assemble()
+    b.solve("fp64")
+    x = b.solution(0)
+    b.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 50)
+    b.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, 0)
+    with pytest.raises(_lib.BemError):
+        b.solve("fp64")
+    with pytest.raises(_lib.BemError) as exc:  # the vectors hold the failed solve's
+        b.solution(0)
+    assert exc.value.code == _lib.BEM_ERR_ARG
+    b.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, -1)
+    b.solve("fp64")
+    assert np.array_equal(b.solution(0), x)
+    b.close()

@@ -385,25 +385,33 @@ int bem_solve(bem_ctx* c, int precision, double rel_tol, int max_iter, double* F
   const int64_t N = c->nsys;
   bem_solve_info st{};
   int rc;
+  // a solve that a wait ended may have written over X, and over A where it factors in place
+  auto timed_out = [&](int e, bool in_place) {
+    if (e == BEM_ERR_TIMEOUT) {
+      c->have_solution = false;
+      if (in_place) c->have_system = false;
+    }
+    return e;
+  };
   BEM_CUDA(c, c->X.alloc(N));
   if (precision == BEM_PREC_FP64) {
     if (c->factored_fp64) return bem_fail(c, BEM_ERR_STATE, "A already factored; assemble again");
     BEM_CUDA(c, c->piv.alloc(N));
     double secs = 0.0;
     rc = bem::lu_factor_fp64(c, c->A.p, c->lda, (int)N, c->piv.p, info, &secs);
-    if (rc) return rc;
+    if (rc) return timed_out(rc, true);
     c->factored_fp64 = true;
     st.factor_seconds = secs;
     st.gflops = secs > 0 ? (2.0 / 3.0) * (double)N * N * N / secs * 1e-9 : 0.0;
     if (*info != 0) return *info;  // DGESV: singular U, no solution
     BEM_CUDA(c, cudaMemcpyAsync(c->X.p, c->FI.p, N * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
     rc = bem::lu_solve_fp64(c, c->A.p, c->lda, (int)N, c->X.p);
-    if (rc) return rc;
+    if (rc) return timed_out(rc, false);
   } else if (precision == BEM_PREC_FP32_IR || precision == BEM_PREC_BF16_IR || precision == BEM_PREC_FP64_IR) {
     rc = bem::solve_mixed(c, precision, rel_tol > 0 ? rel_tol : 1e-12, max_iter > 0 ? max_iter : 50, &st,
                           info);
     if (stats) *stats = st;
-    if (rc) return rc;
+    if (rc) return timed_out(rc, false);
     if (*info != 0) return *info;
   } else {
     return bem_fail(c, BEM_ERR_ARG, "unknown solve precision");

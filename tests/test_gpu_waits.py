@@ -63,6 +63,32 @@ def test_wait_limit_of_a_replayed_factorisation():
     ctx.close()
 
 
+def test_no_result_of_a_failed_solve(cube8_mesh):
+    """The FP64 solve factors A in place: after a wait that ran out neither A nor the solution is
+    taken for one."""
+    from bem3d_elastostatic_b200.api import Quadesth
+
+    q = Quadesth(cube8_mesh)
+    q.precompute_element_geometry()
+    q.ghmat8()
+    x = q.solve_linear_system("fp64-ir")
+    q.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 50)
+    q.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, 0)
+    with pytest.raises(_lib.BemError) as exc:
+        q.solve_linear_system("fp64")
+    assert exc.value.code == _lib.BEM_ERR_TIMEOUT
+    q.set_option(_lib.BEM_OPT_WITHHOLD_PIVOT, -1)
+    q.set_option(_lib.BEM_OPT_WAIT_LIMIT_MS, 2000)
+    for call in (q.reorganize_solution, lambda: q.solve_linear_system("fp64")):
+        with pytest.raises(_lib.BemError) as exc:
+            call()
+        assert exc.value.code == _lib.BEM_ERR_STATE
+    q.ghmat8()
+    y = q.solve_linear_system("fp64")
+    assert np.abs(y - x).max() <= 1e-10 * np.abs(x).max()
+    q.close()
+
+
 # the first panel of a step and the second; one, two and four rows per thread come with the orders
 @pytest.mark.parametrize("precision", ["fp32-ir", "fp64"])
 @pytest.mark.parametrize("ks,pivot", [([3, 1, 4], 0), ([6] * 5 + [2], 45), ([6] * 44, 33)])

@@ -560,7 +560,7 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
     return bfail(b, BEM_ERR_ARG, "batch_solve: precision must be BEM_PREC_FP64 or BEM_PREC_FP32_IR");
   if (max_iter < 1 || max_iter > 30) return bfail(b, BEM_ERR_ARG, "batch_solve: max_iter must be in 1..30");
   for (const auto& D : b->hdev)
-    if (D.N > 25600) return bfail(b, BEM_ERR_TOO_LARGE, "batch_solve: a system of order above 25,600");
+    if (D.N > bem::kMaxOrder) return bfail(b, BEM_ERR_TOO_LARGE, "batch_solve: a system of order above 25,600");
   BB_CUDA(b, cudaSetDevice(b->device));
   int rc;
   const int ns = (int)b->sys.size();

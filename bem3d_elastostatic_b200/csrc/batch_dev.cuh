@@ -7,6 +7,7 @@
 namespace bem {
 
 constexpr int kMaxRhs = 8;  // load cases per system
+constexpr int kMaxOrder = 25600;  // of a system: its pivots and their gather fit in shared memory
 
 struct SysDev {
   int n, ne, N, nrhs;

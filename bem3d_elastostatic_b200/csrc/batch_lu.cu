@@ -892,14 +892,23 @@ __global__ void batch_copy_kernel(const SysDev* __restrict__ sys, const double* 
     F[S.f_off + k] = (T)A[S.a_off + k];
 }
 
+constexpr size_t perm_smem(int n) { return 2 * (size_t)n * sizeof(int); }
+
+// Shared-memory limits, once per device at the most that any batch takes: they are the process's,
+// and a batch that lowered one to its own need would fail another thread's launch.
 template <typename T>
-bool attributes(size_t perm_smem) {
-  return cudaFuncSetAttribute(batch_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)(kTriElems<double> * sizeof(double))) == cudaSuccess &&
-         cudaFuncSetAttribute(batch_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              2 * (int)sizeof(typename UpdateTile<T>::Half)) == cudaSuccess &&
-         cudaFuncSetAttribute(batch_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)perm_smem) ==
-             cudaSuccess;
+bool attributes() {
+  static DeviceOnce set;
+  if (!set.pending()) return true;
+  if (cudaFuncSetAttribute(batch_inv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(kTriElems<double> * sizeof(double))) != cudaSuccess ||
+      cudaFuncSetAttribute(batch_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           2 * (int)sizeof(typename UpdateTile<T>::Half)) != cudaSuccess ||
+      cudaFuncSetAttribute(batch_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)perm_smem(kMaxOrder)) != cudaSuccess)
+    return false;
+  set.mark();
+  return true;
 }
 
 }  // namespace
@@ -921,8 +930,7 @@ int batch_lu_max_order() {
 template <typename T>
 bool batch_solve_enqueue(BatchSolve& b, T* F, double tol, int sweeps) {
   const int maxN = b.N[0], nblk = (maxN + kBlk - 1) / kBlk;
-  const size_t perm_smem = 2 * (size_t)maxN * sizeof(int);
-  if (!attributes<T>(perm_smem)) return false;
+  if (!attributes<T>()) return false;
   if (cudaMemsetAsync(b.info, 0, b.nsys * sizeof(int), b.stream) != cudaSuccess ||
       cudaMemsetAsync(b.conv, 0, b.nsys * sizeof(int), b.stream) != cudaSuccess ||
       cudaMemsetAsync(b.red, 0, (size_t)b.nsys * (3 * kMaxRhs + 1) * sizeof(double), b.stream) != cudaSuccess ||
@@ -940,7 +948,7 @@ bool batch_solve_enqueue(BatchSolve& b, T* F, double tol, int sweeps) {
         b.sys, b.order, b.nsys, F, b.piv, b.info, reinterpret_cast<unsigned*>(b.err + 1));
     ++b.launches;
   }
-  batch_perm_kernel<<<b.nsys, 256, perm_smem, b.stream>>>(b.sys, b.piv, b.perm);
+  batch_perm_kernel<<<b.nsys, 256, perm_smem(maxN), b.stream>>>(b.sys, b.piv, b.perm);
   batch_inv_kernel<T><<<dim3(nblk, 2, b.nsys), kTriThreads, kTriElems<double> * sizeof(double), b.stream>>>(b.sys, F, b.dinv);
   batch_start_kernel<<<dim3((maxN + 255) / 256, b.nsys), 256, 0, b.stream>>>(b.sys, b.FI, b.X, b.R, b.berr);
   b.launches += 3;

@@ -1,0 +1,64 @@
+"""Batches used from several host threads at the same time.  Every result is compared bit for bit
+with the same call made alone."""
+import threading
+
+import numpy as np
+import pytest
+
+from bem3d_elastostatic_b200.mesh import loaded_box
+
+pytestmark = pytest.mark.gpu
+
+
+def _batch(ks, loads=1):
+    from bem3d_elastostatic_b200.api import Batch
+
+    rng = np.random.default_rng(len(ks))
+    b = Batch()
+    for k in ks:
+        b.add(*loaded_box(*rng.uniform(0.7, 1.5, 3), k, 0.3, 1.0, rng.standard_normal((loads, 3))))
+    b.assemble()
+    return b
+
+
+def _run(*jobs):
+    errors = []
+
+    def guarded(job):
+        try:
+            job()
+        except Exception as exc:  # noqa: BLE001 - reported by the main thread
+            errors.append(exc)
+
+    threads = [threading.Thread(target=guarded, args=(job,)) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
+def test_small_batches_beside_a_large_system():
+    """7,206 unknowns, whose pivot gather needs more shared memory than a launch has by default,
+    captured and replayed while another thread captures solves of 78 unknowns."""
+    big = _batch([10])
+    big.solve("fp64", tol=1e-15)
+    ref = big.solution(0)
+    stop = threading.Event()
+
+    def small():
+        while not stop.is_set():
+            b = _batch([1])
+            b.solve("fp64")
+            b.close()
+
+    def large():
+        try:
+            for i in range(12):
+                big.solve("fp64", tol=1e-15 * (1 + i // 2))  # captured anew, replayed
+                assert np.array_equal(big.solution(0), ref)
+        finally:
+            stop.set()
+
+    _run(small, large)
+    big.close()

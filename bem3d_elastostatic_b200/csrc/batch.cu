@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -142,6 +143,7 @@ struct bem_batch {
   double* host_x = nullptr;
   size_t host_cap = 0;
   bool host_valid = false;
+  std::mutex host_lock;  // of the three above: threads may fetch solutions at the same time
   ~bem_batch() {
     if (host_x) cudaFreeHost(host_x);
     if (graph) cudaGraphExecDestroy(graph);
@@ -668,7 +670,9 @@ int bem_batch_solve(bem_batch* b, int precision, double tol, int max_iter, bem_b
 }
 
 int bem_batch_get_solution(bem_batch* b, int i, double* x) {
-  if (!b || !b->factored || i < 0 || i >= (int)b->sys.size() || !x)
+  if (!b) return BEM_ERR_ARG;
+  std::lock_guard<std::mutex> lock(b->host_lock);
+  if (!b->factored || i < 0 || i >= (int)b->sys.size() || !x)
     return bfail(b, BEM_ERR_ARG, "batch_get_solution: bad arguments or no solve");
   const auto& D = b->hdev[i];
   const int64_t nv = b->vec.count / 3;

@@ -1,5 +1,5 @@
-"""Batches used from several host threads at the same time.  Every result is compared bit for bit
-with the same call made alone."""
+"""Batches used from several host threads: different batches at the same time, and the solutions of
+one solved batch.  Every result is compared bit for bit with the same call made alone."""
 import threading
 
 import numpy as np
@@ -62,3 +62,19 @@ def test_small_batches_beside_a_large_system():
 
     _run(small, large)
     big.close()
+
+
+def test_solutions_fetched_by_several_threads():
+    ks = [1, 2, 3, 4] * 4
+    b = _batch(ks, loads=2)
+    b.solve("fp64")
+    ref = [b.solution(i) for i in range(len(ks))]
+    for _ in range(5):
+        b.solve("fp64")  # nothing fetched yet
+
+        def fetch(first):
+            for i in range(first, len(ks), 4):
+                assert np.array_equal(b.solution(i), ref[i])
+
+        _run(*(lambda f=f: fetch(f) for f in range(4)))
+    b.close()

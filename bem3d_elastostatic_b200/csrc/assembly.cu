@@ -133,7 +133,10 @@ constexpr int kTab32 = 12;
 // batch b - 1's.  An mbarrier that a warp arrives at after its additions and waits on before
 // its next ones (not a CTA barrier, which would have all warps integrate and then all add:
 // they slip by up to a batch and one's additions overlap another's integrals).  The wait is
-// bounded; giving it up would cost the order of two roundings, not an entry.
+// bounded by a number of tries.  A warp that gives it up still arrives once a batch, so that no
+// other warp starves, but its arrival may complete the phase of a warp that has not added yet:
+// the additions of this batch, and of those until that warp has caught up, then come in any
+// order.  None is left out; what is lost is that two assemblies agree bit for bit.
 struct BatchOrder {
   unsigned bar;     // mbarrier, one arrival per warp
   unsigned phase;   // of the next wait

@@ -25,6 +25,7 @@
 
 #include "asm_args.cuh"
 #include "common.cuh"
+#include "recip.cuh"
 #include "shape.cuh"
 
 namespace bem {

@@ -100,18 +100,6 @@ struct Kept {
   cudaError_t reserve(size_t n) { return b.count >= n ? cudaSuccess : b.alloc(n); }
 };
 
-// 1 / sqrt(x) from the hardware's approximation of its leading bits and one third-order
-// step: with y (1 + d) = 1 / sqrt(x) and e = 1 - x y^2, y (1 + e/2 + 3/8 e^2) is off by
-// 5/16 e^3, below rounding for the approximation's |e| < 2^-18.  Five FP64 operations; no
-// subnormal or infinite arguments (squared distances).
-__device__ __forceinline__ double rsqrt_h3(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-__device__ __forceinline__ float rsqrt_h3(float x) { return rsqrtf(x); }
-
 // One-time set-up that CUDA keeps per device (kernel attributes, __constant__ tables),
 // tracked per device so that a process driving several GPUs sets up each of them:
 // `static DeviceOnce s; if (s.pending()) { ...; s.mark(); }` with the device current.

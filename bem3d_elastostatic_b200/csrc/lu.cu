@@ -26,6 +26,7 @@
 
 #include "grid_sync.cuh"
 #include "lu.cuh"
+#include "recip.cuh"
 #include "tri_inv.cuh"
 
 namespace bem {
@@ -281,11 +282,7 @@ __device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, in
 // it; the warps past the eighth keep the barriers only.  (One warp with a column per lane and
 // the pivot column by 31 shuffles a step took 14,000 cycles for a diagonally dominant window,
 // this 10,000; a branch around the updates of a warp costs 300 cycles a group.)
-__device__ __forceinline__ float reciprocal_f32(float x) {  // the approximation and one Newton step
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return fmaf(y, fmaf(-x, y, 1.f), y);
-}
+
 // kept out of line: as a select it would be computed for every multiplier
 __device__ __noinline__ float window_quotient(float a, float b) { return a / b; }
 
@@ -338,9 +335,8 @@ __device__ __forceinline__ void window_lu_cta(WindowScratch& ws, float (*D)[kPan
 #pragma unroll
           for (int i = s + 1; i < 4; ++i) u[i] = __shfl_sync(FULL, v[i], pl);
         }
-        const float rp = reciprocal_f32(pv);
-        float l = ct * rp;
-        l = fmaf(fmaf(-l, pv, ct), rp, l);
+        const float rp = reciprocal_newton(pv);
+        float l = corrected_quotient(ct, pv, rp);
         if (!(fabsf(pv) > 1e-30f && fabsf(pv) < 1e30f)) l = window_quotient(ct, pv);  // near the range's ends
         const bool upd = pos > t && pv != 0.f;
         lv[s] = upd ? l : 0.f;

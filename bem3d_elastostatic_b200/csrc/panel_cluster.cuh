@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "lu.cuh"
+#include "recip.cuh"
 
 namespace bem {
 
@@ -100,17 +101,6 @@ __device__ __forceinline__ int warp_pick(unsigned hi, unsigned lo, int pos) {
   }
   return __ffs(at) - 1;
 }
-
-// 1 / x for normal x: the hardware's approximation y of the leading bits and one third-order
-// step, y (1 + e + e^2) with e = 1 - x y (Newton's iteration with one more term).
-__device__ __forceinline__ double reciprocal(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-
-__device__ __forceinline__ float reciprocal(float x) { return __frcp_rn(x); }
 
 // |v| as an ordered integer, NaN as zero
 __device__ __forceinline__ void magnitude(double v, unsigned& hi, unsigned& lo) {
@@ -260,8 +250,7 @@ __device__ __forceinline__ bool panel_steps(const PanelStep& P, PanelSmem<T, LPT
     }
     const T pv = line[0];
     if (live) {
-      // v / pv: the product with the reciprocal and one correction by its remainder; far from
-      // the ends of the exponent range only
+      // v / pv from the reciprocal far from the ends of the exponent range only
       const bool nz = pv != T(0);
       const bool plain = mid_range(pv);
       const T rc = reciprocal(pv);
@@ -269,8 +258,7 @@ __device__ __forceinline__ bool panel_steps(const PanelStep& P, PanelSmem<T, LPT
       T m[LPT];
 #pragma unroll
       for (int q = 0; q < LPT; ++q) {
-        T l = v[q][0] * rc;
-        l = fma(fma(-l, pv, v[q][0]), rc, l);
+        T l = corrected_quotient(v[q][0], pv, rc);
         if (!plain) l = plain_quotient(v[q][0], pv);
         const bool here = !done[q] && pos[q] == p;  // the pivot line: position k from now on
         own_pivot[q] = __ballot_sync(0xffffffffu, here);

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "recip.cuh"
 #include "shape.cuh"
 #include "stress.cuh"
 

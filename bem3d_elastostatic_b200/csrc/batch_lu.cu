@@ -394,7 +394,7 @@ __device__ void cta_getrf(T* A, int64_t lda, int N, int* ipiv, int* info, T* s_a
     for (int j = j0; j < j0 + jb; ++j) {
       double bv = -1.0;
       int bi = INT_MAX;
-      for (int i = j + tid; i < N; i += NT) take_max(bv, bi, fabs((double)A[i + (int64_t)j * lda]), i);
+      for (int i = j + tid; i < N; i += NT) take_max(bv, bi, pivot_size((double)A[i + (int64_t)j * lda]), i);
       for (int off = 16; off > 0; off >>= 1) {
         const double ov = __shfl_xor_sync(0xffffffffu, bv, off);
         const int oi = __shfl_xor_sync(0xffffffffu, bi, off);

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(panel_threads<T>(), 1)
     int bc = INT_MAX, bg = g;
     for (int cc = tid; cc < ncols; cc += blockDim.x) {
       const int cgl = c_beg + cc;
-      if (cgl >= k) better(bv, bc, bg, fabs((double)col[cc * kPitch + t]), cgl, g);
+      if (cgl >= k) better(bv, bc, bg, pivot_size((double)col[cc * kPitch + t]), cgl, g);
     }
     for (int off = 16; off > 0; off >>= 1) {
       const double ov = __shfl_xor_sync(0xffffffffu, bv, off);
@@ -224,7 +224,7 @@ __device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, in
     T pv = D[t][t];
     int p = t;
     if (__any_sync(0xffffffffu, lane > t && fabs((double)ct) > fabs((double)pv))) {
-      double bv = (lane >= t) ? fabs((double)ct) : -1.0;
+      double bv = (lane >= t) ? pivot_size((double)ct) : -1.0;
       int bc = (lane >= t) ? lane : INT_MAX, bg = 0;
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256) window_panel_kernel(T* S, int64_t lda, in
       window_lu_warp<T>(D, s_p, lane);
     } else {
       for (int t = 0; t < w; ++t) {
-        double bv = (lane >= t && lane < w) ? fabs((double)D[lane][t]) : -1.0;
+        double bv = (lane >= t && lane < w) ? pivot_size((double)D[lane][t]) : -1.0;
         int bc = (lane >= t && lane < w) ? lane : INT_MAX, bg = 0;
         for (int off = 16; off > 0; off >>= 1) {
           const double ov = __shfl_xor_sync(0xffffffffu, bv, off);

@@ -56,6 +56,13 @@ int lu_factor_ws(bem_ctx* c, T* S, int64_t lda, int n, int* piv, int* perm, int 
 template <typename T>
 int lu_solve_ws(bem_ctx* c, const T* S, int64_t lda, int n, const int* perm, double* b, double* work);
 
+// The size of a pivot candidate.  NaN counts as zero: it loses every comparison, and a search that
+// met nothing else would end at no line at all.
+__device__ __forceinline__ double pivot_size(double v) {
+  const double a = fabs(v);
+  return a == a ? a : 0.0;
+}
+
 // A pivot or interchange word as its readers take it: after a wait that ran out in the launch that
 // should have written it, it is whatever the buffer held, and the launches up to the host's look at
 // the error word must stay inside the matrix.

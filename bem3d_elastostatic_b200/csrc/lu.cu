@@ -4,7 +4,10 @@
 //
 // One outer step factors an NB-wide panel of T = S^T (NB rows of S) and updates the
 // trailing matrix:
-//   for each 32-wide sub-panel:
+//   FP64, for each 32-wide sub-panel whose lines one cluster holds (panel64.cu): the
+//     cluster's panel, its interchanges with the solve of the panel rows below
+//     (panel_rows_kernel), and their gemm update
+//   otherwise, for each 32-wide sub-panel:
 //     panel_kernel      cooperative launch over the SMs; every CTA holds a slice of
 //                       the sub-panel's S columns in shared memory; per pivot one
 //                       grid barrier (bounded spin) exchanges the per-CTA candidates;
@@ -13,7 +16,11 @@
 //     swap_rows_kernel  applies the sub-panel's swaps to the other rows of the panel
 //                       and to the trailing rows (contiguous column segments)
 //     trsm_small + gemm update of the panel rows below the sub-panel
-//   inv_unit_upper + gemm (TRSM by inverse), then the trailing gemm update.
+//   window-pivoted FP32 panels: the whole diagonal block in one cooperative launch
+//     (panel_coop_kernel), its interchanges (permute_panel_kernel) and both triangles'
+//     inverses (panel_inv.cu), with which the two block TRSMs are one product each
+//   inv_unit_upper + gemm (TRSM by inverse; FP64 and partial pivoting), then the
+//   trailing gemm update.
 #include <cuda.h>
 
 #include <cfloat>
@@ -212,11 +219,9 @@ __global__ void __launch_bounds__(panel_threads<T>(), 1)
 // into registers, updates them there and stores the lane's column back, so the step's
 // shared-memory accesses are independent of one another.  The operations are those of
 // the general loops; the step loop is not unrolled (the warp's code stays in the
-// instruction cache).  s_p[t] receives the local pivot of step t; s_g (nullable, the
-// identity on entry) receives the interchanges composed into a gather: column b of the
-// factored window came from column s_g[b].
+// instruction cache).  s_p[t] receives the local pivot of step t.
 template <typename T>
-__device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, int lane, int* s_g = nullptr) {
+__device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, int lane) {
   constexpr int W = kPanelW;
 #pragma unroll 1
   for (int t = 0; t < W; ++t) {
@@ -237,11 +242,6 @@ __device__ __forceinline__ void window_lu_warp(T (*D)[kPanelW + 1], int* s_p, in
         const T a = D[t][lane];
         D[t][lane] = D[p][lane];
         D[p][lane] = a;
-        if (s_g && lane == 0) {
-          const int gt = s_g[t];
-          s_g[t] = s_g[p];
-          s_g[p] = gt;
-        }
         __syncwarp();
         ct = D[lane][t];
         pv = D[t][t];

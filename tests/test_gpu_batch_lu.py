@@ -51,3 +51,24 @@ def test_systems_added_after_a_solve():
     assert b.solve("fp64")["systems"] == 2
     assert np.abs(b.solution(0) - x0).max() <= 1e-12 * np.abs(x0).max()
     b.close()
+
+
+def test_system_above_the_clusters_capacity():
+    """8,718 unknowns in FP64, above the 8,192 of a cluster: the LU of one CTA per system, for the
+    small system beside it too."""
+    from bem3d_elastostatic_b200.api import Batch
+
+    rng = np.random.default_rng(11)
+    b = Batch()
+    for k in (2, 11):
+        b.add(*loaded_box(*rng.uniform(0.7, 1.5, 3), k, 0.3, 1.0, rng.standard_normal((2, 3))))
+    b.assemble()
+    info = b.solve("fp64")
+    assert info["lu_threads"] == 512 and info["singular"] == 0 and info["max_backward_error"] <= 1e-14
+    for i in range(2):
+        A, F = b.system(i)
+        x = b.solution(i)
+        r = np.abs(F - A @ x).max(0) / (np.abs(A).sum(1).max() * np.abs(x).max(0) + np.abs(F).max(0))
+        assert r.max() <= 1e-14, (i, r)
+    assert b.solve("fp32-ir")["lu_threads"] == 256  # within the 16,384 of FP32
+    b.close()

@@ -62,14 +62,18 @@ __global__ void row_scale_kernel(int n, const unsigned long long* __restrict__ r
 
 // Column scales of the row-scaled matrix and the scaled FP32 copy in one pass per
 // column: a CTA reads column j, reduces its maximum, then converts the column again while
-// it is still in L2.  The grid is sized so that the columns in flight fill half the L2
-// (kColL2 bytes), and each CTA walks its columns in turn.  What bounds it is the 64 bytes
+// it is still in L2, and walks its columns in turn.  What bounds it is the 64 bytes
 // a cycle an SM reads from L2, so the row scales, powers of two, stay in shared memory as
 // their exponents (SMEM; orders whose exponents do not fit read them with the column, which
 // doubles those bytes), and eight 16-byte loads a thread are in flight throughout, the
-// remainder of a column included: 56,454 columns in 7.7 ms, 13.3 ms before.  The FP32
-// copy's padding rows are zero.
-constexpr int kColThreads = 1024;
+// remainder of a column included.  The FP32 copy's padding rows are zero.
+// An SM holds 1,024 of its threads, as four CTAs, two or one: with more CTAs one's loads cover
+// another's reduction, and short columns leave fewer lanes idle, as long as the columns in
+// flight fill no more than half the L2 (kColL2).  Measured (ms at 4,614, 10,374, 18,438,
+// 28,806, 41,478 and 56,454 columns): 256 threads 0.063, 0.232, 0.89, 2.42, 6.5 and 14.3; 512
+// threads 0.072, 0.294, 0.80, 1.93, 5.5 and 11.3; 1,024 threads 0.136, 0.357, 1.08, 1.93, 4.0
+// and 7.7.  A grid of more CTAs than the SMs hold is no faster and at 41,478 takes 5.6.
+constexpr int kColThreads = 1024;  // per SM
 constexpr int kColLoads = 8;  // double2 per thread and turn
 constexpr size_t kColL2 = 64ull << 20;
 constexpr int kColSmem = 220 * 1024;
@@ -77,20 +81,20 @@ constexpr int kColSmem = 220 * 1024;
 __device__ __forceinline__ double pow2_of_field(unsigned f) {
   return __hiloint2double(f == 0 ? 0x00080000 : (int)(f << 20), 0);
 }
-template <bool SMEM>
-__global__ void __launch_bounds__(kColThreads) col_scale_convert_kernel(const double* __restrict__ A, int64_t lda,
-                                                                        int n, const double* __restrict__ rs,
-                                                                        double* __restrict__ cs, float* A32) {
+template <bool SMEM, int NT>
+__global__ void __launch_bounds__(NT) col_scale_convert_kernel(const double* __restrict__ A, int64_t lda, int n,
+                                                               const double* __restrict__ rs,
+                                                               double* __restrict__ cs, float* A32) {
   extern __shared__ __align__(16) unsigned short s_exp[];  // [n rounded up to even]
-  __shared__ double red[kColThreads / 32];
+  __shared__ double red[NT / 32];
   __shared__ double s_c;
   const int t = threadIdx.x;
   if (SMEM) {
-    for (int i = t; i < (n + 1) / 2 * 2; i += kColThreads)
+    for (int i = t; i < (n + 1) / 2 * 2; i += NT)
       s_exp[i] = i < n ? (unsigned short)((__double2hiint(rs[i]) >> 20) & 0x7ff) : 1023;
     __syncthreads();
   }
-  constexpr int STEP = 2 * kColThreads;
+  constexpr int STEP = 2 * NT;
   // rows i and i + 1 of a column, row-scaled; zeros past the matrix
   auto load = [&](const double* a, int i0, double2 (&v)[kColLoads]) {
 #pragma unroll
@@ -127,7 +131,7 @@ __global__ void __launch_bounds__(kColThreads) col_scale_convert_kernel(const do
     __syncthreads();
     if (t == 0) {
       double m = red[0];
-      for (int w = 1; w < kColThreads / 32; ++w) m = fmax(m, red[w]);
+      for (int w = 1; w < NT / 32; ++w) m = fmax(m, red[w]);
       s_c = pow2_scale(m);
       cs[j] = s_c;
     }
@@ -145,6 +149,36 @@ __global__ void __launch_bounds__(kColThreads) col_scale_convert_kernel(const do
     }
     __syncthreads();  // red and s_c are reused by the next column
   }
+}
+
+template <int NT>
+int col_scale_convert_as(bem_ctx* c, int n, int64_t lda) {
+  const int ctas = std::min(n, kColThreads / NT * c->sm_count);
+  const size_t exps = ((size_t)n + 1) / 2 * 2 * sizeof(unsigned short);
+  if constexpr (NT == kColThreads)
+    if (exps > kColSmem) {
+      col_scale_convert_kernel<false, NT>
+          <<<ctas, NT, 0, c->stream>>>(c->A.p, lda, n, c->rowscale.p, c->colscale.p, c->A32.p);
+      return BEM_OK;
+    }
+  static DeviceOnce attr;
+  if (attr.pending()) {
+    BEM_CUDA(c, cudaFuncSetAttribute(col_scale_convert_kernel<true, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kColSmem));
+    attr.mark();
+  }
+  col_scale_convert_kernel<true, NT>
+      <<<ctas, NT, exps, c->stream>>>(c->A.p, lda, n, c->rowscale.p, c->colscale.p, c->A32.p);
+  return BEM_OK;
+}
+
+// colscale and A32 from A and rowscale, by the most CTAs per SM whose columns fit kColL2 (one, if
+// none do)
+int col_scale_convert(bem_ctx* c, int n, int64_t lda) {
+  const size_t columns = kColL2 / ((size_t)lda * sizeof(double));
+  if (columns >= (size_t)4 * c->sm_count) return col_scale_convert_as<kColThreads / 4>(c, n, lda);
+  if (columns >= (size_t)2 * c->sm_count) return col_scale_convert_as<kColThreads / 2>(c, n, lda);
+  return col_scale_convert_as<kColThreads>(c, n, lda);
 }
 
 __global__ void mul_kernel(int n, const double* s, double* x) {
@@ -298,23 +332,7 @@ int solve_mixed(bem_ctx* c, int precision, double rel_tol, int max_iter, bem_sol
     BEM_LAUNCH_CHECK(c);
     row_scale_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(n, rmax, c->rowscale.p);
     BEM_LAUNCH_CHECK(c);
-    const int64_t col_ctas =
-        std::max<int64_t>(1, std::min<int64_t>({(int64_t)n, (int64_t)(kColL2 / ((size_t)lda * sizeof(double))),
-                                                (int64_t)2 * c->sm_count}));
-    const size_t exps = ((size_t)n + 1) / 2 * 2 * sizeof(unsigned short);
-    if (exps <= kColSmem) {
-      static DeviceOnce attr;
-      if (attr.pending()) {
-        BEM_CUDA(c, cudaFuncSetAttribute(col_scale_convert_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kColSmem));
-        attr.mark();
-      }
-      col_scale_convert_kernel<true><<<(unsigned)col_ctas, kColThreads, exps, c->stream>>>(
-          c->A.p, lda, n, c->rowscale.p, c->colscale.p, c->A32.p);
-    } else {
-      col_scale_convert_kernel<false><<<(unsigned)col_ctas, kColThreads, 0, c->stream>>>(
-          c->A.p, lda, n, c->rowscale.p, c->colscale.p, c->A32.p);
-    }
+    if ((rc = col_scale_convert(c, n, lda))) return rc;
   } else if (dbl) {
     BEM_CUDA(c, cudaMemcpyAsync(c->A64f.p, c->A.p, (size_t)lda * n * sizeof(double), cudaMemcpyDeviceToDevice,
                                 c->stream));

@@ -9,6 +9,12 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+# and the last order of four CTAs per SM, the first of two
+@pytest.mark.parametrize("n", [14144, 14145])
+def test_row_units_change_nothing_where_the_ctas_change(n):
+    test_row_units_change_nothing(n)
+
+
 @pytest.mark.parametrize("n", [2, 33, 1001, 2047, 2048, 2049, 16387])
 def test_row_units_change_nothing(n):
     from bem3d_elastostatic_b200.api import solve_system

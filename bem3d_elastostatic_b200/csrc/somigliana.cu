@@ -292,7 +292,7 @@ constexpr int kChunkDoubles = kChunk * kGp * kRec;  // one staged chunk of eleme
 
 // Far pass: CTA (x, y) sums the element chunks [nchunks y / S, nchunks (y + 1) / S) of S =
 // gridDim.y shares at the points [256 x, 256 (x + 1)), one per thread, into part[y][9][l].
-// The shares give a call with few points enough CTAs (a single tile used to run on one SM)
+// The shares give a call with few points enough CTAs (a single tile alone fills one SM)
 // and even out the last wave.  Bound: FP64 pipe, 83 % active (16 warps per SM at 126
 // registers).  100,003 points x 960 elements: 49.6 -> 21.2 ms by SomAcc::add; 3,001 points x
 // 484 elements: 8.3 -> 0.35 ms, the rest by the shares.  counters[0] accumulates the table points evaluated (far

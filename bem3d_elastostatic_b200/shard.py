@@ -77,7 +77,8 @@ def internal_points_sharded(q, points: Optional[np.ndarray] = None, kelvin_consi
     """compute_internal_points over all ranks of ``group``: ``q`` is this rank's
     :class:`~bem3d_elastostatic_b200.api.Quadesth` holding the solved system (every
     rank solved the same system).  Returns (u, sigma, prin, vm) for all points on
-    every rank, identical to a single-GPU call."""
+    every rank, equal to a single-GPU call up to rounding (how a point's sums are split
+    depends on the number of points in the call)."""
     m = q.mesh
     if points is None:
         points = np.stack([m.cx, m.cy, m.cz], axis=1)

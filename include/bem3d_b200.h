@@ -256,7 +256,7 @@ typedef struct {
   double solve_seconds;        /* device time of the whole solve (factor + sweeps) */
   int lu_threads;              /* CTA size of the LU: 256 panel by panel over all systems, 512
                                   one CTA per system (a system above the cluster's capacity) */
-  float lu_ms_256, lu_ms_512;  /* no longer measured: 0 */
+  float lu_ms_256, lu_ms_512;  /* always 0 */
 } bem_batch_info;
 
 int bem_batch_create(bem_batch** batch, int device);

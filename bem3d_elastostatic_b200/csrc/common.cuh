@@ -194,6 +194,7 @@ struct bem_ctx {
   bem::DBuf<float> A32;
   bem::DBuf<int> piv;
   bem::DBuf<int> perm;  // gather form of the pivots of the latest factorisation (solve side)
+  bem::DBuf<int> dgesv_perm;  // perm's place during a bem_dgesv, whose factors are the caller's
   bem::DBuf<double> work;
   bem::DBuf<float> work32;
   bem::DBuf<unsigned int> sync;

@@ -424,6 +424,22 @@ int bem_solve(bem_ctx* c, int precision, double rel_tol, int max_iter, double* F
   return BEM_OK;
 }
 
+namespace {
+// The gather of the context's own factors, which a later transposed solve takes, set aside while a
+// bem_dgesv computes its own.
+struct OwnGather {
+  bem_ctx* c;
+  explicit OwnGather(bem_ctx* ctx) : c(ctx) { swap(); }
+  OwnGather(const OwnGather&) = delete;
+  OwnGather& operator=(const OwnGather&) = delete;
+  ~OwnGather() { swap(); }
+  void swap() {
+    std::swap(c->perm.p, c->dgesv_perm.p);
+    std::swap(c->perm.count, c->dgesv_perm.count);
+  }
+};
+}  // namespace
+
 int bem_dgesv(bem_ctx* c, int n, int nrhs, double* A, int lda, int* ipiv, double* B, int ldb, int* info) {
   if (!c || !A || !ipiv || !B || !info || n <= 0 || nrhs < 0 || lda < n || ldb < n)
     return bem_fail(c, BEM_ERR_ARG, "dgesv: bad arguments");
@@ -443,6 +459,7 @@ int bem_dgesv(bem_ctx* c, int n, int nrhs, double* A, int lda, int* ipiv, double
     BEM_CUDA(c, cudaMemcpy2DAsync(dB, ld * sizeof(double), B, (size_t)ldb * sizeof(double), n * sizeof(double),
                                   nrhs, cudaMemcpyHostToDevice, c->stream));
   double secs = 0.0;
+  const OwnGather own(c);
   int rc = bem::lu_factor_fp64(c, dA, ld, n, dp, info, &secs);
   if (rc) return rc;
   if (*info == 0)

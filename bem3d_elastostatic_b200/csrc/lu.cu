@@ -2078,10 +2078,10 @@ __device__ __forceinline__ bool tile_wait(unsigned bar, unsigned parity, unsigne
 //   either block.  Publication to publication: one poll, 32 multiply-adds and two barriers.
 // One CTA barrier per tile: the partial sums alternate between two buffers.  A tile costs 1,024
 // cycles of conversions to FP64 (a quarter of the multiply-add's rate).
-// A wait that runs out, for a block or for a tile, ends the whole CTA at its next barrier: the
-// tiles not used yet stay the only ones under way, each half of the ring keeps the phase it was
-// armed for, and thread 0 waits for them (again within the limit) before the CTA leaves.  A sweep
-// that finds the status word set (the other sweep of the solve gave up) asks for no tile.
+// A wait that runs out records the error; a poll then ends the sweep as soon as it has to wait
+// (what is summed and published up to there is of no account).  From the first tile on that thread
+// 0 has not seen arrive it asks for none, so that no half of the ring is armed again before its
+// phase is complete, and before the CTA leaves it waits for the tiles under way.
 // Measured, a sweep of 56,000 unknowns: 1.29 ms (4.9 TB/s), of 18,432: 0.28 ms (1.9 us a block);
 // with tiles two deep in registers and inverse and product between poll and publication 2.36 and
 // 0.41 ms.  Loading the lead block or the inverse when it is needed costs 1 us a block each;
@@ -2104,7 +2104,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   __shared__ __align__(16) double ys[NB];
   __shared__ double red[2][4][NB];
   __shared__ __align__(8) unsigned long long s_bar[2];
-  __shared__ int s_abort, s_lost[2];  // a block, by `par` a tile, that did not come
+  __shared__ int s_abort;
   const int t = threadIdx.x, lane = t & 31, G = gridDim.x, g = blockIdx.x;
   const int nblk = (n + NB - 1) / NB;
   const int rl = t & (NB - 1), q = t >> 7;  // this thread's row; its columns are 32 q .. 32 q + 31
@@ -2155,17 +2155,13 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   };
 #pragma unroll
   for (int u = 0; u < 32; ++u) m[u] = 0.0;
-  bool over = false;  // thread 0: given up before it began
   if (t == 0) {
     tile_bar_init(bar_s);
     tile_bar_init(bar_s + 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    s_abort = s_lost[0] = s_lost[1] = 0;
-    over = *((volatile int*)status) != 0;
-    if (!over) {
-      fill();
-      fill();
-    }
+    s_abort = 0;
+    fill();
+    fill();
   }
   if (g < nblk) stage(g);
   const int nown = (g < nblk) ? (nblk - 1 - g) / G + 1 : 0;
@@ -2174,7 +2170,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     wacc[i] = (k0 + r < n) ? b[k0 + r] : 0.0;
   }
   cp_async_all();
-  if (__syncthreads_or(over)) return;
+  __syncthreads();
 
   auto inv_product = [&](int s) {  // this thread's share of Dinv w for step s
     const double* D = Di + lane;
@@ -2207,9 +2203,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 
   if (g == 0) publish(0, inv_product(0));
   int used = 0;
-  bool lost = false;  // a tile that did not come (the same in all threads)
+  bool filling = true;
 #pragma unroll 1
-  for (int s = 0; s + 1 < nblk && !lost; ++s) {
+  for (int s = 0; s + 1 < nblk; ++s) {
     const int s2 = first(s);
     if (s2 >= nblk) break;  // no rows left to update
     const int cb = min(NB, n - bidx(s) * NB);
@@ -2237,7 +2233,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 #pragma unroll 1
     for (; sx < nblk; sx += G) {
       const int h = used & 1;
-      if (!tile_wait(bar_s + 8 * h, (used >> 1) & 1, wait_ns, status)) s_lost[par] = 1;
+      const bool here = tile_wait(bar_s + 8 * h, (used >> 1) & 1, wait_ns, status);
+      if (!here) atomicCAS(status, 0, BEM_ERR_TIMEOUT);
+      filling &= here;
       const float* p = ring + h * NB * NB + 32 * q * NB + rl;
       double a = 0.0;
 #pragma unroll
@@ -2248,21 +2246,16 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
       }
       red[par][q][rl] = a;
       __syncthreads();
-      lost = s_lost[par] != 0;  // written again two barriers from here at the earliest
-      if (lost) {
-        if (t == 0) atomicCAS(status, 0, BEM_ERR_TIMEOUT);
-        break;
-      }
       ++used;
-      if (t == 0) fill();  // the tile just read makes room
+      if (t == 0 && filling) fill();  // the tile just read makes room
       if (t < NB)
         wacc[((sx - g) / G) * NB + t] -= (red[par][0][t] + red[par][1][t]) + (red[par][2][t] + red[par][3][t]);
       par ^= 1;
     }
   }
   cp_async_all();
-  if (t == 0)  // the tiles under way when the sweep was given up
-    for (int k = used; k < asked; ++k) tile_wait(bar_s + 8 * (k & 1), (k >> 1) & 1, wait_ns, nullptr);
+  if (t == 0)  // copies under way when the sweep was given up
+    for (int k = max(0, asked - 2); k < asked; ++k) tile_wait(bar_s + 8 * (k & 1), (k >> 1) & 1, wait_ns, nullptr);
 }
 
 // ---- the transposed solve: S^T x = b with the same factors --------------------------

@@ -21,6 +21,8 @@
 //   Residual: one CTA per 128 rows, the columns streamed once for all load cases.
 // Measured on 96 boxes of 78 to 2,598 unknowns with eight load cases: FP32 LU 155 -> 14.2 ms, ten
 // sweeps 42 -> 6.8 ms, residuals 15.9 -> 2.7 ms.
+#include <math_constants.h>
+
 #include <algorithm>
 #include <climits>
 
@@ -820,7 +822,7 @@ __global__ void __launch_bounds__(256) batch_residual_kernel(const SysDev* __res
       xv = fabs(X[at]);
       rv = bv - (acc[q] + s_h[r][q]);
       R[at] = rv;
-      rv = fabs(rv);
+      rv = rv == rv ? fabs(rv) : CUDART_INF;  // fmax would pass over a NaN
       bv = fabs(bv);
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -838,7 +840,8 @@ __global__ void __launch_bounds__(256) batch_residual_kernel(const SysDev* __res
   if (lane == 0) max_into(m + 3 * kMaxRhs, asum);
 }
 
-// backward error max_r ||R_r|| / (||A|| ||X_r|| + ||B_r||) (infinity norms); conv = 1 once it is
+// backward error max_r ||R_r|| / (||A|| ||X_r|| + ||B_r||) (infinity norms; infinite where a residual
+// is NaN); conv = 1 once it is
 // <= tol, 2 once a sweep gains less than 10 %; the maxima are cleared for the next pass
 __global__ void batch_conv_kernel(const SysDev* __restrict__ sys, int nsys, double* __restrict__ red,
                                   double* __restrict__ berr, int* __restrict__ conv, const int* __restrict__ info,
@@ -849,7 +852,7 @@ __global__ void batch_conv_kernel(const SysDev* __restrict__ sys, int nsys, doub
   double be = 0.0;
   for (int q = 0; q < sys[s].nrhs; ++q) {
     const double den = m[3 * kMaxRhs] * m[kMaxRhs + q] + m[2 * kMaxRhs + q];
-    be = fmax(be, den > 0.0 ? m[q] / den : 0.0);
+    be = fmax(be, m[q] == CUDART_INF ? CUDART_INF : den > 0.0 ? m[q] / den : 0.0);
   }
   for (int q = 0; q < 3 * kMaxRhs + 1; ++q) m[q] = 0.0;
   const double prev = berr[s];

@@ -59,3 +59,26 @@ def test_nan_entries_dgesv(n):
     X = dgesv(A, b, ctx=ctx)[2]
     assert np.abs(A @ X[:, 0] - b).max() <= 1e-13 * np.abs(A).sum(1).max() * np.abs(X).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp32-ir", "fp64"])
+def test_batch_with_a_collapsed_element(precision):
+    """A system whose normals are 0 / 0 does not count as converged; the one beside it does."""
+    from bem3d_elastostatic_b200.api import Batch, SolverFailure
+    from bem3d_elastostatic_b200.mesh import loaded_box
+
+    b = Batch()
+    good, bad = loaded_box(1.0, 1.0, 1.0, 3, 0.3), loaded_box(1.0, 1.0, 1.0, 2, 0.3)
+    nodes = bad[0].kconec[:, 0] - 1
+    for v in (bad[0].x, bad[0].y, bad[0].z):
+        v[nodes] = v[nodes[0]]
+    b.add(*good)
+    b.add(*bad)
+    b.assemble()
+    try:
+        b.solve(precision, tol=1e-13)
+        assert b.info["max_backward_error"] == np.inf
+    except SolverFailure:  # a zero pivot among the NaN
+        assert b.info["singular"] == 1
+    assert b.info["converged"] == 1
+    b.close()
